@@ -13,7 +13,7 @@ Three kinds, each through the package's public entry points:
 
 A pass runs a stretch of an exponentiation from a dense residue and reads the
 registers back, as a program does at a checkpoint or at the end of a test.
-Bases are even, log-uniform in [b_lo, b_hi].  The digits the engine returns
+Bases are even, log-uniform in [b_lo, b_hi] (or uniform, where the case says so).  The digits the engine returns
 stand for a residue but are not unique (balanced, a unit of carry may stay
 unreduced), so a pass returns them in the one canonical form, digits in [0, b).
 """
@@ -58,7 +58,7 @@ def listed():
         {"name": "batch n12 x 102", "kind": "batch", "n": 12, "count": 102, "b_lo": 1024, "b_hi": 2_000_000_000, "blocks": 2},
         {"name": "batch n14 x 38", "kind": "batch", "n": 14, "count": 38, "b_lo": 1024, "b_hi": 2_000_000_000, "blocks": 2},
         # the batched search at the headline size
-        {"name": "batch n16 x 64", "kind": "batch", "n": 16, "count": 64, "b_lo": 1_000_000, "b_hi": 100_000_000, "blocks": 2},
+        {"name": "batch n16 x 64", "kind": "batch", "n": 16, "count": 64, "b_lo": 1_000_000, "b_hi": 100_000_000, "blocks": 2, "uniform": True},
         # a serving pool, bases up to the size's limit
         {"name": "batch n18 x 8", "kind": "batch", "n": 18, "count": 8, "b_lo": 50_000_000, "b_hi": 1_000_000_000, "blocks": 2},
     ]
@@ -82,7 +82,7 @@ def draw(rng):
         most = min(130 if n <= 13 else 64, MOST_DIGIT_SQUARINGS // (BLOCK << n))
         count = max(1, int(math.exp(rng.uniform(0.0, math.log(most + 1)))))
         blocks = max(1, min(2, MOST_DIGIT_SQUARINGS // (count * BLOCK << n)))
-        return {"kind": kind, "n": n, "count": count, "b_lo": lo, "b_hi": hi, "blocks": blocks}
+        return {"kind": kind, "n": n, "count": count, "b_lo": lo, "b_hi": hi, "blocks": blocks, "uniform": rng.random() < 0.5}
     n = rng.randint(12, 16) if kind == "prime" else rng.randint(12, 23)
     lo, hi = _bases_range(rng, n)
     steps = min(int(math.exp(rng.uniform(math.log(200), math.log(1000)))), MOST_DIGIT_SQUARINGS >> n)
@@ -90,8 +90,9 @@ def draw(rng):
 
 
 def _bases(case, rng, count):
-    b = np.exp(rng.uniform(math.log(case["b_lo"]), math.log(case["b_hi"]), count))
-    return [max(case["b_lo"], int(x)) & ~1 for x in b]
+    lo, hi = case["b_lo"], case["b_hi"]
+    b = rng.uniform(lo, hi, count) if case.get("uniform") else np.exp(rng.uniform(math.log(lo), math.log(hi), count))
+    return [max(lo, int(x)) & ~1 for x in b]
 
 
 def _inputs(case, seed):
