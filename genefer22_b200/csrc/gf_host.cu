@@ -535,17 +535,16 @@ int sm_count()
 template <int SET, int LOGN>
 void small_t(const Args &a, int grid, cudaStream_t s, bool prep)
 {
-	using S = SmallShape<SET, LOGN, false>;
-	using SS = SmallShape<SET, LOGN, true>;
-	if (prep)
+	using L = SmallLaunch<SET, LOGN, false>;
+	using LS = SmallLaunch<SET, LOGN, true>;
+	if (prep) set_smem(k_small<SET, LOGN, false>, L::SMEM);
+	if constexpr (LS::PSPLIT)
 	{
-		set_smem(k_small<SET, LOGN, false>, S::SMEM);
-		set_smem(k_small<SET, LOGN, true>, SS::SMEM);
-		return;
+		// fewer tests than SMs: plane-split passes (more warps per test)
+		if (prep) set_smem(k_small<SET, LOGN, true>, LS::SMEM);
+		else if (grid < sm_count()) { launch_pdl(k_small<SET, LOGN, true>, dim3(grid), dim3(LS::T), LS::SMEM, s, a); return; }
 	}
-	// fewer tests than SMs: plane-split passes (more warps per test)
-	if (SS::PSPLIT && (grid < sm_count())) launch_pdl(k_small<SET, LOGN, true>, dim3(grid), dim3(SS::T), SS::SMEM, s, a);
-	else launch_pdl(k_small<SET, LOGN, false>, dim3(grid), dim3(S::T), S::SMEM, s, a);
+	if (!prep) launch_pdl(k_small<SET, LOGN, false>, dim3(grid), dim3(L::T), L::SMEM, s, a);
 }
 
 template <int SET>
@@ -838,13 +837,6 @@ constexpr int PLAN_PACKED = 200;  // plan codes 200 + lr: packed digits, four-st
 constexpr int PLAN_PACKED_SIX = 300;   // plan codes 300 + lr2: packed digits, six-step of n - 1
 
 constexpr int PLAN_CLUSTER = 1;   // plan code of the cluster-resident squaring
-// A batch of at most this many tests of size 12..14 squares on the cluster
-// plan by default: one test on 8 or 16 SMs instead of one (a lone n = 12, 13,
-// 14 test on one CTA 15.4, 31.3, 62.4 us per squaring; on the cluster now
-// 6.6, 8.2, 10.3, graph replay on one B200); larger batches fill the SMs with
-// one CTA per test.
-constexpr size_t CLUSTER_MAX_TESTS = 4;
-
 bool plan_valid(int n, int lr)
 {
 	if (lr > PLAN_PACKED_SIX)
@@ -880,6 +872,24 @@ int default_plan(int n)
 	if (n <= 16) return n - 12;
 	static const int lr2[24] = { 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 3, 3, 4, 4, 5, 6, 7 };
 	return PLAN_SIX + lr2[n];
+}
+
+// Default plan of `count` tests at n = 12..14 (nset: tests per prime set), from
+// the time of one batch squaring under every plan (graph replay on one B200, us).
+// The cluster plan (8 or 16 CTAs a test) until its CTAs crowd the SMs or the
+// 16-CTA clusters a second wave: n = 12, single-CTA -> cluster, 48 tests 15.0 ->
+// 9.8, 52 tests 15.1 -> 15.5; n = 13, four-step -> cluster, 12 tests 15.1 -> 9.2,
+// 16 tests 16.2 -> 17.4; n = 14 7 tests 15.8 -> 10.3, 8 tests 16.1 -> 20.4.  Then one
+// CTA per test at n = 12 (102 tests: 15.2, four-step 26.3); at n = 13, 14 one CTA's
+// transform is long, and the four-step plan (lr = 3) spreads it: n = 13 51 tests
+// 31.2 -> 22.4, n = 14 38 tests 62.8 -> 29.0.  Wide batches of one prime set keep one
+// CTA per test (n = 13 128 tests 31.3, four-step 35.9; n = 14 62.6, 61.0).
+int default_small_plan(int n, size_t count, const int (&nset)[2])
+{
+	static const size_t cluster_max[3] = { 48, 12, 7 };
+	if (count <= cluster_max[n - 12]) return PLAN_CLUSTER;
+	if ((n >= 13) && ((count < 64) || ((nset[0] > 0) && (nset[1] > 0)))) return 3;
+	return 0;
 }
 
 // The default packs a batch of at least this many tests whose bases all fit
@@ -931,10 +941,9 @@ struct gfc_batch
 	uint32_t *d_err = nullptr;
 	std::vector<TestDesc> h_desc;
 	std::vector<uint32_t *> ebits;
-	int nset[2] = { 0, 0 }, offset[2] = { 0, 0 };   // tests per prime set; d_tests lists set 0 first
+	int nset[2] = { 0, 0 };       // tests per prime set
 	int pending = -1;             // register whose segment carries are not yet absorbed (four-step)
-	uint64_t sets_version = 0;    // bumped when a test changes prime set (per-set launches change)
-	bool tests_sorted = true;     // d_tests lists the tests by prime set (only the single-CTA plan needs it)
+	uint64_t sets_version = 0;    // bumped when a test changes prime set (the single-CTA kernel is chosen by the sets present)
 	int cluster = 0;              // 1 when squarings use k_cluster (shape by n), else 0
 	int six = 0;                  // lr2 of a six-step plan (columns 2^4 x 2^lr2, lr = 4 + lr2), else 0
 	bool packed = false;          // prime set 2, two digits per coefficient, transform of N/2 (lr of that)
@@ -949,7 +958,7 @@ struct gfc_batch
 	uint64_t res_bits = 0;        // exponent bits each slot can hold (0: not reserved)
 	size_t res_words = 0;         // device words per slot
 	uint32_t *d_eres = nullptr;   // count x res_words exponent words
-	char *h_pin = nullptr;        // pinned: per slot [TestDesc | int64 pos | res_words words], then tests[], one
+	char *h_pin = nullptr;        // pinned: per slot [TestDesc | int64 pos | res_words words], then one
 	size_t pin_slot = 0;          // bytes per slot in h_pin
 	std::vector<cudaEvent_t> slot_ev;   // recorded after a slot's staged copies were enqueued
 
@@ -977,7 +986,7 @@ struct gfc_graph
 	cudaGraphExec_t exec = nullptr;
 	uint64_t kernels = 0;         // kernel nodes recorded
 	uint64_t sets_version = 0;    // batch's sets_version at capture
-	bool per_set = false;         // recorded per-prime-set launches (single-CTA plan)
+	bool per_set = false;         // recorded the kernel of the prime sets present (single-CTA plan)
 	~gfc_graph()
 	{
 		cudaSetDevice(device);
@@ -1085,16 +1094,20 @@ Args make_args(const gfc_batch &bt)
 	return a;
 }
 
-// Single-CTA kernels: one launch per prime set present (tests sorted by set).
-void launch_small(const gfc_batch &bt, const Args &a0, cudaStream_t s, bool prep)
+// Single-CTA kernel: one launch for all tests.
+void launch_small(const gfc_batch &bt, const Args &a, cudaStream_t s, bool prep)
 {
-	for (int set = 0; set < 2; ++set)
+	const int grid = static_cast<int>(bt.count);
+	if (prep)      // every variant: an admission may change the sets present
 	{
-		if (bt.nset[set] == 0) continue;
-		Args a = a0;
-		a.tests = bt.d_tests + bt.offset[set];
-		if (set == 0) small_set<0>(bt.n, a, bt.nset[set], s, prep); else small_set<1>(bt.n, a, bt.nset[set], s, prep);
+		small_set<0>(bt.n, a, grid, s, true);
+		small_set<1>(bt.n, a, grid, s, true);
+		small_set<SMALL_BOTH>(bt.n, a, grid, s, true);
+		return;
 	}
+	if (bt.nset[1] == 0) small_set<0>(bt.n, a, grid, s, false);
+	else if (bt.nset[0] == 0) small_set<1>(bt.n, a, grid, s, false);
+	else small_set<SMALL_BOTH>(bt.n, a, grid, s, false);
 }
 
 // Cluster-resident squarings: one persistent launch over all tests.
@@ -1445,7 +1458,6 @@ gfc_batch *batch_create(const uint32_t *b, size_t count, uint32_t n, size_t num_
 		bt->set[i] = s;
 		bt->nset[s]++;
 	}
-	bt->offset[0] = 0; bt->offset[1] = bt->nset[0];
 	apply_plan(*bt, default_plan(bt->n));
 
 	GFC_CK(cudaSetDevice(device));
@@ -1473,10 +1485,8 @@ gfc_batch *batch_create(const uint32_t *b, size_t count, uint32_t n, size_t num_
 
 	bt->h_desc.resize(count);
 	bt->ebits.assign(count, nullptr);
-	std::vector<int32_t> tests;
-	for (int s = 0; s < 2; ++s)
-		for (size_t i = 0; i < count; ++i)
-			if (bt->set[i] == s) tests.push_back(static_cast<int32_t>(i));
+	std::vector<int32_t> tests(count);
+	for (size_t i = 0; i < count; ++i) tests[i] = static_cast<int32_t>(i);
 	for (size_t i = 0; i < count; ++i)
 	{
 		TestDesc &d = bt->h_desc[i];
@@ -1502,8 +1512,7 @@ gfc_batch *batch_create(const uint32_t *b, size_t count, uint32_t n, size_t num_
 		set_packed(*bt, true);
 		apply_plan(*bt, default_packed_plan(bt->n, count));
 	}
-	else if ((bt->n >= 12) && (bt->n <= SMALL_MAX_LOGN) && (count <= CLUSTER_MAX_TESTS))
-		apply_plan(*bt, PLAN_CLUSTER);
+	else if ((bt->n >= 12) && (bt->n <= SMALL_MAX_LOGN)) apply_plan(*bt, default_small_plan(bt->n, count, bt->nset));
 	prepare_plan(*bt);
 	return bt.release();
 }
@@ -1637,8 +1646,7 @@ PinSlot pin_slot(const gfc_batch &bt, size_t test)
 			 reinterpret_cast<uint32_t *>(p + sizeof(TestDesc) + sizeof(int64_t)) };
 }
 
-int32_t *pin_tests(const gfc_batch &bt) { return reinterpret_cast<int32_t *>(bt.h_pin + bt.count * bt.pin_slot); }
-int32_t *pin_one(const gfc_batch &bt) { return pin_tests(bt) + bt.count; }
+int32_t *pin_one(const gfc_batch &bt) { return reinterpret_cast<int32_t *>(bt.h_pin + bt.count * bt.pin_slot); }
 
 void op_reserve(gfc_batch &bt, uint64_t max_bits)
 {
@@ -1649,12 +1657,12 @@ void op_reserve(gfc_batch &bt, uint64_t max_bits)
 	const size_t slot = (sizeof(TestDesc) + sizeof(int64_t) + 4 * words + 15) & ~size_t(15);
 	bt.d_eres = static_cast<uint32_t *>(dev_alloc(bt.device, bt.count * words * sizeof(uint32_t), bt.stream));
 	GFC_CK(cudaMemsetAsync(bt.d_eres, 0, bt.count * words * sizeof(uint32_t), bt.stream));
-	bt.h_pin = static_cast<char *>(pinned_get(bt.count * slot + (bt.count + 1) * sizeof(int32_t)));
+	bt.h_pin = static_cast<char *>(pinned_get(bt.count * slot + sizeof(int32_t)));
 	if (bt.h_pin == nullptr) fail(GFC_ERR_CUDA, "reserve: no page-locked host memory for the staging");
 	bt.res_words = words;
 	bt.pin_slot = slot;
 	*pin_one(bt) = 1;
-	bt.slot_ev.assign(bt.count + 1, nullptr);          // one per slot, then one for the tests list
+	bt.slot_ev.assign(bt.count, nullptr);
 	for (cudaEvent_t &e : bt.slot_ev) GFC_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
 	GFC_CK(cudaStreamSynchronize(bt.stream));
 	bt.res_bits = max_bits;
@@ -1698,29 +1706,10 @@ void op_admit(gfc_batch &bt, size_t test, uint32_t b, const uint32_t *words, uin
 	materialize(bt);
 	if (s != bt.set[test])
 	{
-		// prime-set order of the per-set launches (single-CTA plan)
 		bt.sets_version++;
 		bt.nset[bt.set[test]]--;
 		bt.set[test] = s;
 		bt.nset[s]++;
-		bt.offset[0] = 0; bt.offset[1] = bt.nset[0];
-		if (bt.lr == 0)
-		{
-			// the per-set launches read the tests in prime-set order; the
-			// staging of the previous order is rewritten after its copy ran
-			// (a wait for the block in flight when two admissions of one
-			// window change sets)
-			staging_free(bt, bt.count);
-			int32_t *tl = pin_tests(bt);
-			size_t k = 0;
-			for (int q = 0; q < 2; ++q)
-				for (size_t i = 0; i < bt.count; ++i)
-					if (bt.set[i] == q) tl[k++] = static_cast<int32_t>(i);
-			GFC_CK(cudaMemcpyAsync(bt.d_tests, tl, bt.count * sizeof(int32_t), cudaMemcpyHostToDevice, bt.stream));
-			GFC_CK(cudaEventRecord(bt.slot_ev[bt.count], bt.stream));
-			prepare_plan(bt);
-		}
-		else bt.tests_sorted = false;   // every other launch covers all tests in any order
 	}
 	bt.b[test] = b;
 	TestDesc &d = bt.h_desc[test];
@@ -1750,15 +1739,6 @@ void set_plan_checked(gfc_batch &bt, int lr)
 	GFC_CK(cudaStreamSynchronize(bt.stream));
 	if (packed != bt.packed) set_packed(bt, packed);
 	apply_plan(bt, lr);
-	if ((bt.lr == 0) && !bt.tests_sorted)
-	{
-		std::vector<int32_t> tests;
-		for (int q = 0; q < 2; ++q)
-			for (size_t i = 0; i < bt.count; ++i)
-				if (bt.set[i] == q) tests.push_back(static_cast<int32_t>(i));
-		GFC_CK(cudaMemcpy(bt.d_tests, tests.data(), bt.count * sizeof(int32_t), cudaMemcpyHostToDevice));
-		bt.tests_sorted = true;
-	}
 	prepare_plan(bt);
 }
 
@@ -2097,11 +2077,6 @@ GFC_API int gfc_batch_assign(gfc_batch *bt, size_t test, uint32_t b)
 		bt->b[test] = b;
 		bt->set[test] = s;
 		bt->nset[s]++;
-		bt->offset[0] = 0; bt->offset[1] = bt->nset[0];
-		std::vector<int32_t> tests;
-		for (int k = 0; k < 2; ++k)
-			for (size_t i = 0; i < bt->count; ++i)
-				if (bt->set[i] == k) tests.push_back(static_cast<int32_t>(i));
 		if (bt->packed && !packed_ok(b, bt->n)) fail(GFC_ERR_RANGE, "assign: base outside the range of packed digits");
 		TestDesc &d = bt->h_desc[test];
 		d.b = b;
@@ -2114,8 +2089,6 @@ GFC_API int gfc_batch_assign(gfc_batch *bt, size_t test, uint32_t b)
 			d.pk = pack_constants(b);
 		}
 		GFC_CK(cudaMemcpy(bt->d_desc + test, &d, sizeof(TestDesc), cudaMemcpyHostToDevice));
-		GFC_CK(cudaMemcpy(bt->d_tests, tests.data(), bt->count * sizeof(int32_t), cudaMemcpyHostToDevice));
-		bt->tests_sorted = true;
 		prepare_plan(*bt);
 	});
 }

@@ -222,8 +222,9 @@ int gfc_batch_set_all(gfc_batch *bt, size_t reg, const int32_t *in);
  * otherwise single-CTA up to n = 14,
  * four-step at n = 15, 16 (lr = n - 12), six-step above (103 at n = 17, 18,
  * 104 at n = 19, 20, 105 at n = 21, 106 at n = 22, 107 at n = 23; a lone test at
- * n = 19 too, packed or not, and at n = 12..14 the cluster plan): the fastest plans measured
- * on one B200.
+ * n = 19 too, packed or not); at n = 12..14 up to 48, 12 and 7 tests the cluster
+ * plan, and at n = 13, 14 four-step (lr = 3) for fewer than 64 tests and for
+ * batches of both widths: the fastest plans measured on one B200.
  * gfc_batch_plan reads the current plan. */
 int gfc_batch_set_plan(gfc_batch *bt, int lr);
 int gfc_batch_plan(const gfc_batch *bt);
