@@ -14,9 +14,10 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libgfcuda.so")
-SOURCES = [os.path.join(CSRC, f) for f in ("gf_host.cu", "gf_probe.cu", "gf_gint.cpp", "gf_server.cpp",
+INSTANCES = [f"gf_inst_{g}.cu" for g in ("small", "cluster_short", "cluster_long", "col", "colr", "row", "row_pair", "mid", "pcol")]
+SOURCES = [os.path.join(CSRC, f) for f in ("gf_host.cu", "gf_probe.cu", *INSTANCES, "gf_gint.cpp", "gf_server.cpp",
                                            "gf_server_cuda.cpp")]
-DEPS = SOURCES + [os.path.join(CSRC, f) for f in ("gf_arith.cuh", "gf_ntt.cuh", "gf_kernels.cuh", "gf_server.h")] + \
+DEPS = SOURCES + [os.path.join(CSRC, f) for f in ("gf_arith.cuh", "gf_ntt.cuh", "gf_kernels.cuh", "gf_inst.cuh", "gf_server.h")] + \
     [os.path.join(ROOT, "include", "gfcuda.h")]
 
 NVCC_FLAGS = [
@@ -24,6 +25,7 @@ NVCC_FLAGS = [
     "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC,-fvisibility=hidden",
     "-shared",
+    "--threads", "0",       # the sources in parallel
 ]
 
 

@@ -17,7 +17,19 @@
 #include <vector>
 
 #include "../../include/gfcuda.h"
-#include "gf_kernels.cuh"
+#include "gf_inst.cuh"
+
+namespace gfc {
+GFC_INST_SMALL(extern template __global__)
+GFC_INST_CLUSTER_SHORT(extern template __global__)
+GFC_INST_CLUSTER_LONG(extern template __global__)
+GFC_INST_COL(extern template __global__)
+GFC_INST_COLR(extern template __global__)
+GFC_INST_ROW(extern template __global__)
+GFC_INST_ROW_PAIR(extern template __global__)
+GFC_INST_MID(extern template __global__)
+GFC_INST_PCOL(extern template __global__)
+}  // namespace gfc
 
 using namespace gfc;
 
@@ -76,9 +88,16 @@ void launch_pdl(K *kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t s, c
 	after_launch();
 }
 
+// The form of an unpacked kernel that holds set 3's body, or the one without.
+template <class K>
+void launch_s3(K *with, K *without, dim3 grid, dim3 block, size_t smem, cudaStream_t s, const Args &a)
+{
+	launch_pdl(a.s3 ? with : without, grid, block, smem, s, a);
+}
+
 // ------------------------------------------------------------------ roots
 
-// Prime slots: set 0 = slots 0,1; set 1 = slots 2,3,4.
+// Prime slots: set 0 = slots 0,1; set 1 = slots 2,3,4 (set 3 its first two).
 const uint32_t kPrime[5] = { PrimeSet<0>::p[0], PrimeSet<0>::p[1], PrimeSet<1>::p[0], PrimeSet<1>::p[1], PrimeSet<1>::p[2] };
 
 inline uint32_t mulmod_h(uint32_t a, uint32_t b, uint32_t p) { return static_cast<uint32_t>((static_cast<uint64_t>(a) * b) % p); }
@@ -405,17 +424,23 @@ const TwistTables &get_twist(DeviceTables &t, bool packed, int lr)
 
 // Exact range: with |digit| <= D = b/2 + 1 every coefficient of a product of
 // two resting registers is at most N D^2 in absolute value; the centred CRT
-// of set S is exact when N D^2 < floor(M_S / 2).
-int choose_set(uint32_t b, int n)
+// of set S is exact when N D^2 < floor(M_S / 2).  The first of sets 3 (with
+// `s3`), 0 and 1 that holds it.
+int choose_set(uint32_t b, int n, bool s3)
 {
 	const u128 D = b / 2 + 1;
 	const u128 bound = (u128(1) << n) * D * D;
+	const u128 M3 = u128(PrimeSet<3>::p[0]) * PrimeSet<3>::p[1];
 	const u128 M0 = u128(PrimeSet<0>::p[0]) * PrimeSet<0>::p[1];
 	const u128 M1 = u128(PrimeSet<1>::p[0]) * PrimeSet<1>::p[1] * PrimeSet<1>::p[2];
+	if (s3 && (bound < M3 / 2)) return 3;
 	if (bound < M0 / 2) return 0;
 	if (bound < M1 / 2) return 1;
 	return -1;
 }
+
+// Primes of an unpacked set.
+int set_width(int set) { return (set == 1) ? 3 : 2; }
 
 // Root tables of prime set 2 for the packed transform of 2^np points
 // (cached under key -np).
@@ -484,9 +509,9 @@ PackK pack_constants(uint32_t b)
 // Constants of the fused CRT + carry (gf_arith.cuh, CarryK) for base b.
 CarryK carry_constants(uint32_t b, int set)
 {
-	const u128 T = (set == 0) ? u128(PrimeSet<0>::p[0]) : u128(PrimeSet<1>::p[0]) * PrimeSet<1>::p[1];
+	const u128 T = (set == 0) ? u128(PrimeSet<0>::p[0]) : ((set == 3) ? u128(PrimeSet<3>::p[0]) : u128(PrimeSet<1>::p[0]) * PrimeSet<1>::p[1]);
 	const u128 M = (set == 0) ? u128(PrimeSet<0>::p[0]) * PrimeSet<0>::p[1]
-							  : u128(PrimeSet<1>::p[0]) * PrimeSet<1>::p[1] * PrimeSet<1>::p[2];
+							  : u128(PrimeSet<1>::p[0]) * PrimeSet<1>::p[1] * ((set == 3) ? 1u : PrimeSet<1>::p[2]);
 	CarryK k{};
 	k.b = b;
 	k.h = b / 2;
@@ -535,16 +560,18 @@ int sm_count()
 template <int SET, int LOGN>
 void small_t(const Args &a, int grid, cudaStream_t s, bool prep)
 {
-	using L = SmallLaunch<SET, LOGN, false>;
-	using LS = SmallLaunch<SET, LOGN, true>;
-	if (prep) set_smem(k_small<SET, LOGN, false>, L::SMEM);
+	// n = 10, 11 have the kernel of any set only
+	constexpr int ST = (LOGN >= 12) ? SET : ANY_SET;
+	using L = SmallLaunch<ST, LOGN, false>;
+	using LS = SmallLaunch<ST, LOGN, true>;
+	if (prep) set_smem(k_small<ST, LOGN, false>, L::SMEM);
 	if constexpr (LS::PSPLIT)
 	{
 		// fewer tests than SMs: plane-split passes (more warps per test)
-		if (prep) set_smem(k_small<SET, LOGN, true>, LS::SMEM);
-		else if (grid < sm_count()) { launch_pdl(k_small<SET, LOGN, true>, dim3(grid), dim3(LS::T), LS::SMEM, s, a); return; }
+		if (prep) set_smem(k_small<ST, LOGN, true>, LS::SMEM);
+		else if (grid < sm_count()) { launch_pdl(k_small<ST, LOGN, true>, dim3(grid), dim3(LS::T), LS::SMEM, s, a); return; }
 	}
-	if (!prep) launch_pdl(k_small<SET, LOGN, false>, dim3(grid), dim3(L::T), L::SMEM, s, a);
+	if (!prep) launch_pdl(k_small<ST, LOGN, false>, dim3(grid), dim3(L::T), L::SMEM, s, a);
 }
 
 template <int SET>
@@ -578,18 +605,18 @@ void col_t(bool inv, const Args &a, int grid_y, cudaStream_t s, bool prep)
 	{
 		// R <= 16: a thread owns a column (register kernels)
 		using S = ColRegShape<LR>;
-		if (prep) { set_smem(k_colr_inv<LR>, S::SMEM); return; }
+		if (prep) { set_smem(k_colr_inv<LR, true>, S::SMEM); set_smem(k_colr_inv<LR, false>, S::SMEM); return; }
 		const size_t cols = size_t(1) << (a.n - LR);
 		if (split_cols(cols, grid_y, 8))
 		{
 			const dim3 grid(static_cast<unsigned>(cols / CS_T), static_cast<unsigned>(grid_y));
-			if (inv) launch_pdl(k_colr_inv_s<LR>, grid, dim3(WMAX * CS_T), 0, s, a);
-			else launch_pdl(k_colr_fwd_s<LR>, grid, dim3(WMAX * CS_T), 0, s, a);
+			if (inv) launch_s3(k_colr_inv_s<LR, true>, k_colr_inv_s<LR, false>, grid, dim3(WMAX * CS_T), 0, s, a);
+			else launch_s3(k_colr_fwd_s<LR, true>, k_colr_fwd_s<LR, false>, grid, dim3(WMAX * CS_T), 0, s, a);
 			return;
 		}
 		const dim3 grid(static_cast<unsigned>(cols / COLR_THREADS), static_cast<unsigned>(grid_y));
-		if (inv) launch_pdl(k_colr_inv<LR>, grid, dim3(COLR_THREADS), S::SMEM, s, a);
-		else launch_pdl(k_colr_fwd<LR>, grid, dim3(COLR_THREADS), 0, s, a);
+		if (inv) launch_s3(k_colr_inv<LR, true>, k_colr_inv<LR, false>, grid, dim3(COLR_THREADS), S::SMEM, s, a);
+		else launch_s3(k_colr_fwd<LR, true>, k_colr_fwd<LR, false>, grid, dim3(COLR_THREADS), 0, s, a);
 	}
 	else
 	{
@@ -624,7 +651,12 @@ void row_t(const Args &a, int grid_y, cudaStream_t s, bool prep, int planes)
 {
 	using S = RowShape<LC>;
 	const size_t smem = size_t(S::PC) * 4;          // one plane per CTA
-	if (prep) { set_smem(k_row<LC>, smem); set_smem(k_row2<LC>, 2 * smem); set_smem(k_rowp<LC>, 2 * smem); return; }
+	if (prep)
+	{
+		set_smem(k_row<LC, true>, smem); set_smem(k_row<LC, false>, smem);
+		set_smem(k_row2<LC>, 2 * smem); set_smem(k_rowp<LC>, 2 * smem);
+		return;
+	}
 	// A pair per CTA halves the grid: it pays for rows of 8192 points (512
 	// threads, one CTA per SM) and from 1024 CTAs of single rows; below, the
 	// single rows run in parallel instead (two packed tests at n = 17, 128 row
@@ -659,7 +691,7 @@ void row_t(const Args &a, int grid_y, cudaStream_t s, bool prep, int planes)
 		return;
 	}
 	const dim3 grid((1u << (a.n - LC)) * static_cast<unsigned>(planes), static_cast<unsigned>(grid_y));
-	launch_pdl(k_row<LC>, grid, dim3(row_threads(LC)), smem, s, a);
+	launch_s3(k_row<LC, true>, k_row<LC, false>, grid, dim3(row_threads(LC)), smem, s, a);
 }
 
 void launch_row(int lc, const Args &a, int grid_y, cudaStream_t s, bool prep, int planes = 3)
@@ -720,11 +752,11 @@ void launch_pcol(int lr, bool inv, const Args &a, int grid_y, cudaStream_t s, bo
 // allows 16-CTA clusters and returns in *max_out how many clusters fit on the
 // device at once; otherwise launches a persistent grid of
 // min(ntests, max_active) clusters over the tests a.tests[0 .. ntests-1].
-template <int LQ, int LC>
-void cluster_t(const Args &a, int ntests, int max_active, cudaStream_t s, bool prep, int *max_out)
+template <int LQ, int LC, int SET>
+void cluster_set(const Args &a, int ntests, int max_active, cudaStream_t s, bool prep, int *max_out)
 {
 	using S = ClusterShape<LQ, LC>;
-	auto kern = k_cluster<LQ, LC>;
+	auto kern = k_cluster<LQ, LC, SET>;
 	cudaLaunchConfig_t cfg = {};
 	cudaLaunchAttribute at[1];
 	at[0].id = cudaLaunchAttributeClusterDimension;
@@ -740,7 +772,7 @@ void cluster_t(const Args &a, int ntests, int max_active, cudaStream_t s, bool p
 		int m = 0;
 		GFC_CK(cudaOccupancyMaxActiveClusters(&m, kern, &cfg));
 		if (m < 1) fail(GFC_ERR_CUDA, "cluster plan: no cluster of this size fits on the device");
-		*max_out = m;
+		*max_out = std::min(*max_out, m);
 		return;
 	}
 	const int ncl = (ntests < max_active) ? ntests : max_active;
@@ -759,22 +791,33 @@ void cluster_t(const Args &a, int ntests, int max_active, cudaStream_t s, bool p
 	after_launch();
 }
 
+// `set`: 0 (sets 0 and 1), 3 (set 3 only; n = 12..14), or ANY_SET.
+template <int LQ, int LC>
+void cluster_t(const Args &a, int ntests, int max_active, int set, cudaStream_t s, bool prep, int *max_out)
+{
+	if (prep || (set == 0)) cluster_set<LQ, LC, 0>(a, ntests, max_active, s, prep, max_out);
+	if constexpr (LC <= 10)
+		if (prep || (set == 3)) cluster_set<LQ, LC, 3>(a, ntests, max_active, s, prep, max_out);
+	if (prep || (set == ANY_SET)) cluster_set<LQ, LC, ANY_SET>(a, ntests, max_active, s, prep, max_out);
+}
+
 // Cluster shape by size: n = 12..14 with plane-split passes on rows of
 // 2^(n-LQ) (eight CTAs at n = 12, 16 at n = 13, 14), n = 15..17 on 2..16 CTAs
 // with rows of 2^13.  One test on one B200 (graph replay, us per squaring),
 // 8 -> 16 CTAs with the balanced row schedule: n = 12 6.75 -> 9.95 (2^8-point
 // rows of two 16-point passes leave half of the threads idle), n = 13 8.80 ->
 // 8.31; n = 14 13.04 (eight CTAs, earlier schedule) -> 10.40.
-void launch_cluster_n(int n, const Args &a, int ntests, int max_active, cudaStream_t s, bool prep, int *max_out)
+void launch_cluster_n(int n, const Args &a, int ntests, int max_active, int set, cudaStream_t s, bool prep, int *max_out)
 {
+	if (prep) *max_out = 1 << 30;
 	switch (n)
 	{
-		case 12: cluster_t<3, 9>(a, ntests, max_active, s, prep, max_out); break;
-		case 13: cluster_t<4, 9>(a, ntests, max_active, s, prep, max_out); break;
-		case 14: cluster_t<4, 10>(a, ntests, max_active, s, prep, max_out); break;
-		case 15: cluster_t<2, 13>(a, ntests, max_active, s, prep, max_out); break;
-		case 16: cluster_t<3, 13>(a, ntests, max_active, s, prep, max_out); break;
-		case 17: cluster_t<4, 13>(a, ntests, max_active, s, prep, max_out); break;
+		case 12: cluster_t<3, 9>(a, ntests, max_active, set, s, prep, max_out); break;
+		case 13: cluster_t<4, 9>(a, ntests, max_active, set, s, prep, max_out); break;
+		case 14: cluster_t<4, 10>(a, ntests, max_active, set, s, prep, max_out); break;
+		case 15: cluster_t<2, 13>(a, ntests, max_active, set, s, prep, max_out); break;
+		case 16: cluster_t<3, 13>(a, ntests, max_active, set, s, prep, max_out); break;
+		case 17: cluster_t<4, 13>(a, ntests, max_active, set, s, prep, max_out); break;
 		default: fail(GFC_ERR_ARG, "cluster plan needs 12 <= n <= 17");
 	}
 }
@@ -805,8 +848,8 @@ void midr_t(bool inv, const Args &a, int grid_y, cudaStream_t s, bool prep, int 
 	const size_t C = size_t(1) << (a.n - MID_LR1 - LR2);
 	const dim3 grid(static_cast<unsigned>((size_t(1) << MID_LR1) * size_t(planes) * (C / MIDR_THREADS)),
 					static_cast<unsigned>(grid_y));
-	if (inv) launch_pdl(k_midr<LR2, true>, grid, dim3(MIDR_THREADS), 0, s, a);
-	else launch_pdl(k_midr<LR2, false>, grid, dim3(MIDR_THREADS), 0, s, a);
+	if (inv) launch_s3(k_midr<LR2, true, true>, k_midr<LR2, true, false>, grid, dim3(MIDR_THREADS), 0, s, a);
+	else launch_s3(k_midr<LR2, false, true>, k_midr<LR2, false, false>, grid, dim3(MIDR_THREADS), 0, s, a);
 }
 
 void launch_mid(int lr2, bool inv, const Args &a, int grid_y, cudaStream_t s, bool prep, int planes = 3)
@@ -823,8 +866,8 @@ void launch_mid(int lr2, bool inv, const Args &a, int grid_y, cudaStream_t s, bo
 			const size_t C = size_t(1) << (a.n - MID_LR1 - 6);
 			const dim3 grid(static_cast<unsigned>((size_t(1) << MID_LR1) * size_t(planes) * (C / MIDP_COLS)),
 							static_cast<unsigned>(grid_y));
-			if (inv) launch_pdl(k_midp<true>, grid, dim3(MIDP_THREADS), 0, s, a);
-			else launch_pdl(k_midp<false>, grid, dim3(MIDP_THREADS), 0, s, a);
+			if (inv) launch_s3(k_midp<true, true>, k_midp<true, false>, grid, dim3(MIDP_THREADS), 0, s, a);
+			else launch_s3(k_midp<false, true>, k_midp<false, false>, grid, dim3(MIDP_THREADS), 0, s, a);
 			break;
 		}
 		case 7: mid_t<7>(inv, a, grid_y, s, prep, planes); break;
@@ -837,6 +880,7 @@ constexpr int PLAN_PACKED = 200;  // plan codes 200 + lr: packed digits, four-st
 constexpr int PLAN_PACKED_SIX = 300;   // plan codes 300 + lr2: packed digits, six-step of n - 1
 
 constexpr int PLAN_CLUSTER = 1;   // plan code of the cluster-resident squaring
+
 bool plan_valid(int n, int lr)
 {
 	if (lr > PLAN_PACKED_SIX)
@@ -884,11 +928,11 @@ int default_plan(int n)
 // transform is long, and the four-step plan (lr = 3) spreads it: n = 13 51 tests
 // 31.2 -> 22.4, n = 14 38 tests 62.8 -> 29.0.  Wide batches of one prime set keep one
 // CTA per test (n = 13 128 tests 31.3, four-step 35.9; n = 14 62.6, 61.0).
-int default_small_plan(int n, size_t count, const int (&nset)[2])
+int default_small_plan(int n, size_t count, const int (&nset)[4])
 {
 	static const size_t cluster_max[3] = { 48, 12, 7 };
 	if (count <= cluster_max[n - 12]) return PLAN_CLUSTER;
-	if ((n >= 13) && ((count < 64) || ((nset[0] > 0) && (nset[1] > 0)))) return 3;
+	if ((n >= 13) && ((count < 64) || ((nset[1] > 0) && (nset[1] < static_cast<int>(count))))) return 3;
 	return 0;
 }
 
@@ -929,6 +973,7 @@ struct gfc_batch
 	size_t N = 0, count = 0, num_regs = 0;
 	std::vector<uint32_t> b;
 	std::vector<int> set;
+	bool s3 = false;              // a base of the batch was in set 3's range when it was made: its tests may use it
 	int lr = 0;
 	std::shared_ptr<DeviceTables> tab;
 	void *mem = nullptr;
@@ -941,7 +986,7 @@ struct gfc_batch
 	uint32_t *d_err = nullptr;
 	std::vector<TestDesc> h_desc;
 	std::vector<uint32_t *> ebits;
-	int nset[2] = { 0, 0 };       // tests per prime set
+	int nset[4] = { 0, 0, 0, 0 }; // tests per prime set (0, 1, 3)
 	int pending = -1;             // register whose segment carries are not yet absorbed (four-step)
 	uint64_t sets_version = 0;    // bumped when a test changes prime set (the single-CTA kernel is chosen by the sets present)
 	int cluster = 0;              // 1 when squarings use k_cluster (shape by n), else 0
@@ -1090,8 +1135,17 @@ Args make_args(const gfc_batch &bt)
 	a.lr = bt.lr;
 	a.num_regs = static_cast<int>(bt.num_regs);
 	a.pdl_graph = (bt.packed && (bt.six <= 5)) ? 1 : 0;
+	a.s3 = (!bt.packed && bt.s3) ? 1 : 0;
 	a.ntests = static_cast<uint32_t>(bt.count);
 	return a;
+}
+
+// The prime set of every test of the batch, or ANY_SET.
+int common_set(const gfc_batch &bt)
+{
+	for (int set : { 0, 1, 3 })
+		if (bt.nset[set] == static_cast<int>(bt.count)) return set;
+	return ANY_SET;
 }
 
 // Single-CTA kernel: one launch for all tests.
@@ -1102,25 +1156,32 @@ void launch_small(const gfc_batch &bt, const Args &a, cudaStream_t s, bool prep)
 	{
 		small_set<0>(bt.n, a, grid, s, true);
 		small_set<1>(bt.n, a, grid, s, true);
-		small_set<SMALL_BOTH>(bt.n, a, grid, s, true);
+		small_set<3>(bt.n, a, grid, s, true);
+		small_set<ANY_SET>(bt.n, a, grid, s, true);
 		return;
 	}
-	if (bt.nset[1] == 0) small_set<0>(bt.n, a, grid, s, false);
-	else if (bt.nset[0] == 0) small_set<1>(bt.n, a, grid, s, false);
-	else small_set<SMALL_BOTH>(bt.n, a, grid, s, false);
+	switch (common_set(bt))
+	{
+		case 0: small_set<0>(bt.n, a, grid, s, false); break;
+		case 1: small_set<1>(bt.n, a, grid, s, false); break;
+		case 3: small_set<3>(bt.n, a, grid, s, false); break;
+		default: small_set<ANY_SET>(bt.n, a, grid, s, false);
+	}
 }
 
 // Cluster-resident squarings: one persistent launch over all tests.
 void launch_cluster(gfc_batch &bt, const Args &a, cudaStream_t s)
 {
-	launch_cluster_n(bt.n, a, static_cast<int>(bt.count), bt.cluster_max, s, false, nullptr);
+	// set 3's own kernel only where a graph is refused once a test has changed set
+	const int set = !bt.s3 ? 0 : (((bt.lr == 0) && (common_set(bt) == 3)) ? 3 : ANY_SET);
+	launch_cluster_n(bt.n, a, static_cast<int>(bt.count), bt.cluster_max, set, s, false, nullptr);
 }
 
 // Raises shared-memory limits of the kernels the current plan uses.
 // Whether a six-step plan twists in its middle pass (every row then reads
 // the same C - 1 roots): where one direction of the row-pass root tables
 // (32 B per point of the packed transform, 24 B per point with a test on
-// the three-prime set, else 8 B) reaches 32 MB, and only for the register
+// the three-prime set, 16 B with one on two 31-bit primes, else 8 B) reaches 32 MB, and only for the register
 // middle passes of 2^3 .. 2^5 rows.  (The tables of every prime are built,
 // so a later admission on another prime set stays exact.)  Measured per squaring on one
 // B200 (graph replay, twist off -> on): packed n = 21 plan 305 76.0 -> 73.6
@@ -1134,6 +1195,7 @@ bool twist_pays(const gfc_batch &bt)
 	size_t per_point = 8;
 	if (bt.packed) per_point = 32;
 	else if (bt.nset[1] > 0) per_point = 24;
+	else if (bt.nset[3] > 0) per_point = 16;
 	const size_t points = size_t(1) << (bt.packed ? bt.n - 1 : bt.n);
 	return per_point * points >= (size_t(32) << 20);
 }
@@ -1145,7 +1207,7 @@ void prepare_plan(gfc_batch &bt)
 		bt.twist = bt.packed ? &get_twist(*bt.tabp, true, bt.lr) : &get_twist(*bt.tab, false, bt.lr);
 	Args a{};
 	a.n = bt.n;
-	if (bt.cluster > 0) launch_cluster_n(bt.n, a, 0, 0, nullptr, true, &bt.cluster_max);
+	if (bt.cluster > 0) launch_cluster_n(bt.n, a, 0, 0, ANY_SET, nullptr, true, &bt.cluster_max);
 	if (bt.packed)
 	{
 		launch_pcol(bt.six ? MID_LR1 : bt.lr, true, a, 0, nullptr, true);
@@ -1453,10 +1515,11 @@ gfc_batch *batch_create(const uint32_t *b, size_t count, uint32_t n, size_t num_
 	for (size_t i = 0; i < count; ++i)
 	{
 		if ((b[i] < 8) || (b[i] >= (1u << 31))) fail(GFC_ERR_ARG, "base b must satisfy 8 <= b < 2^31");
-		const int s = choose_set(b[i], static_cast<int>(n));
+		const int s = choose_set(b[i], static_cast<int>(n), true);
 		if (s < 0) fail(GFC_ERR_RANGE, "(b, n) is outside the exact range of the RNS prime sets");
 		bt->set[i] = s;
 		bt->nset[s]++;
+		bt->s3 |= (s == 3);
 	}
 	apply_plan(*bt, default_plan(bt->n));
 
@@ -1700,7 +1763,7 @@ void op_admit(gfc_batch &bt, size_t test, uint32_t b, const uint32_t *words, uin
 	if (bt.res_bits == 0) fail(GFC_ERR_STATE, "admit: reserve the batch first (gfc_batch_reserve)");
 	if ((nbits == 0) || (nbits > bt.res_bits)) fail(GFC_ERR_ARG, "admit: need 1 <= nbits <= the reserved bits");
 	if ((b < 8) || (b >= (1u << 31))) fail(GFC_ERR_ARG, "admit: base b must satisfy 8 <= b < 2^31");
-	const int s = choose_set(b, bt.n);
+	const int s = choose_set(b, bt.n, bt.s3);
 	if (s < 0) fail(GFC_ERR_RANGE, "admit: (b, n) is outside the exact range of the RNS prime sets");
 	if (bt.packed && !packed_ok(b, bt.n)) fail(GFC_ERR_RANGE, "admit: base outside the range of packed digits");
 	materialize(bt);
@@ -1873,7 +1936,7 @@ GFC_API size_t gfc_get_mem_size(const gfc_transform *t) { return (t == nullptr) 
 GFC_API size_t gfc_get_cache_size(const gfc_transform *t)
 {
 	if (t == nullptr) return 0;
-	return (t->set[0] == 0 ? 2 : 3) * t->N * sizeof(uint32_t) + t->N * sizeof(int32_t);
+	return set_width(t->set[0]) * t->N * sizeof(uint32_t) + t->N * sizeof(int32_t);
 }
 
 GFC_API size_t gfc_context_size(const gfc_transform *t, size_t num_regs)
@@ -1920,7 +1983,7 @@ GFC_API int gfc_read_context(gfc_transform *t, const void *buf, size_t size, siz
 GFC_API int gfc_width(const gfc_transform *t)
 {
 	if (t == nullptr) return GFC_ERR_ARG;
-	return t->packed ? 4 : (t->set[0] == 0 ? 2 : 3);
+	return t->packed ? 4 : set_width(t->set[0]);
 }
 
 GFC_API int gfc_sync(gfc_transform *t)
@@ -2028,8 +2091,8 @@ GFC_API int gfc_batch_set_async(gfc_batch *bt, size_t test, size_t reg, const in
 GFC_API int gfc_width_for(uint32_t b, uint32_t n)
 {
 	if ((b < 8) || (b >= (1u << 31)) || (n < 8) || (n > 23)) return GFC_ERR_ARG;
-	const int s = choose_set(b, static_cast<int>(n));
-	return (s < 0) ? GFC_ERR_RANGE : ((s == 0) ? 2 : 3);
+	const int s = choose_set(b, static_cast<int>(n), true);
+	return (s < 0) ? GFC_ERR_RANGE : set_width(s);
 }
 
 GFC_API int gfc_packed_range(uint32_t b, uint32_t n)
@@ -2067,7 +2130,7 @@ GFC_API int gfc_batch_assign(gfc_batch *bt, size_t test, uint32_t b)
 		check_test(*bt, test);
 		no_capture(*bt);
 		if ((b < 8) || (b >= (1u << 31))) fail(GFC_ERR_ARG, "assign: base b must satisfy 8 <= b < 2^31");
-		const int s = choose_set(b, bt->n);
+		const int s = choose_set(b, bt->n, bt->s3);
 		if (s < 0) fail(GFC_ERR_RANGE, "assign: (b, n) is outside the exact range of the RNS prime sets");
 		cudaSetDevice(bt->device);
 		materialize(*bt);
@@ -2240,7 +2303,7 @@ GFC_API int gfc_batch_widths(const gfc_batch *bt, int32_t *w)
 {
 	return guard([&] {
 		GFC_NULLCHK(bt); GFC_NULLCHK(w);
-		for (size_t i = 0; i < bt->count; ++i) w[i] = bt->packed ? 4 : ((bt->set[i] == 0) ? 2 : 3);
+		for (size_t i = 0; i < bt->count; ++i) w[i] = bt->packed ? 4 : set_width(bt->set[i]);
 	});
 }
 
@@ -2435,7 +2498,7 @@ GFC_API int gfc_square_noalloc(const int32_t *in, int32_t *out, uint32_t b, uint
 				fail(GFC_ERR_ARG, "square_noalloc: in and out must be equal or disjoint");
 		}
 		if ((b < 8) || (b >= (1u << 31))) fail(GFC_ERR_ARG, "square_noalloc: base b must satisfy 8 <= b < 2^31");
-		const int set = choose_set(b, static_cast<int>(n));
+		const int set = choose_set(b, static_cast<int>(n), false);
 		if (set < 0) fail(GFC_ERR_RANGE, "square_noalloc: (b, n) is outside the exact range of the RNS prime sets");
 		std::lock_guard<std::mutex> lock(g_na_mu);
 		GFC_CK(cudaSetDevice(device));

@@ -51,7 +51,7 @@ struct TestDesc
 	CarryK ck;              // constants of the fused CRT + carry for this b
 	PackK pk;               // packed-digit constants (set 2)
 	uint32_t b;
-	int32_t set;            // prime set: 0 (W = 2), 1 (W = 3), 2 (W = 4, packed digits)
+	int32_t set;            // prime set: 0 or 3 (W = 2), 1 (W = 3), 2 (W = 4, packed digits)
 };
 
 // Root tables per prime (entries as load_twiddles reads them: one word in
@@ -72,15 +72,19 @@ struct Args
 	const int32_t *tests;   // indices of the tests this launch serves
 	int64_t *pos;           // per-test current exponent bit index
 	uint32_t *err;          // error flags (bit 0: carry not absorbed)
-	Tables tab[3];          // root tables of prime sets 0, 1 (length N) and 2 (length N/2)
+	Tables tab[3];          // root tables of prime sets 0, 1 (and 3; length N) and 2 (length N/2): tab_of
 	int n, lr;              // log2 N, log2 R (four-step)
 	int num_regs, src, dst; // registers
 	int op, dup_mode, count, j;  // operation, dup source, squarings (k_small), squaring index in block
 	int fix;                // four-step column-forward: register src has pending segment carries
 	int pdl_graph;          // host only: graph-captured launches keep programmatic edges
+	int s3;                 // host only: the batch may hold tests of set 3 (kernels with S3)
 	int twist;              // six-step: the middle pass twists, every row transform has base 1
 	uint32_t ntests;        // tests of the batch (0: unchecked); the guard of test_ok
 };
+
+// Index of a prime set's root tables: set 3 uses set 1's.
+__host__ __device__ constexpr int tab_of(int set) { return (set == 3) ? 1 : set; }
 
 template <int SET, int PL>
 using ZS = Zp<PrimeSet<SET>::p[PL], PrimeSet<SET>::P31>;
@@ -95,6 +99,26 @@ __device__ __forceinline__ void for_planes(F &&f)
 }
 
 
+
+// Kernels of unpacked launches come with and without S3: a batch none of whose
+// tests was on set 3 when it was made keeps its tests on sets 0 and 1, and its
+// kernels hold the bodies of those only.  (With the third body in every kernel
+// ptxas took more registers or another schedule: one B200, 3-prime batches of 64
+// at n = 16 125.3 -> 127.5 us per squaring, at n = 15 66.8 -> 68.7, a lone packed
+// test at n = 20 43.0 -> 44.4.)  Set 3 runs set 1's row and middle passes on its
+// first two planes.
+constexpr int ANY_SET = 4;       // template argument of kernels that take each test's set as it comes
+
+__device__ __forceinline__ int set_planes(int set) { return (set == 1) ? 3 : 2; }
+
+// f(integral_constant<SET>) for the set of a test of an unpacked launch.
+template <bool S3, class F>
+__device__ __forceinline__ void by_set(int set, F &&f)
+{
+	if (set == 0) f(std::integral_constant<int, 0>{});
+	else if (!S3 || (set == 1)) f(std::integral_constant<int, 1>{});
+	else f(std::integral_constant<int, 3>{});
+}
 
 __device__ __forceinline__ bool exp_bit(const uint32_t *ebits, int64_t i)
 {
@@ -584,7 +608,7 @@ __device__ __forceinline__ void small_body(const Args &a, int t, const TestDesc 
 	constexpr int D = N / T0;          // digits per owner thread (multiple of SEG)
 	static_assert(D % SEG == 0, "digits per thread");
 	int64_t *const sc = reinterpret_cast<int64_t *>(sm + S::W * PN);
-	const Tables &tab = a.tab[SET];
+	const Tables &tab = a.tab[tab_of(SET)];
 	const int tid = threadIdx.x;
 	const bool owner = (tid < T0);     // the other threads join the transform passes only
 	using MP = RowMap<LOGN>;
@@ -663,16 +687,15 @@ __device__ __forceinline__ void small_body(const Args &a, int t, const TestDesc 
 	if ((tid == 0) && (a.op == OP_SQUARE) && (a.dup_mode == DUP_BITS)) a.pos[t] -= done;
 }
 
-// One CTA per test of prime set SET, or with SET = SMALL_BOTH of the set of its
+// One CTA per test of prime set SET, or with SET = ANY_SET of the set of its
 // test: threads and shared memory are then those of the three-prime set (the
-// threads past a two-prime test's own only join the barriers).  A batch of both
-// sets runs in one launch: with a launch per set the second waited for the
-// first (102 tests at n = 12, one B200: 31.6 -> 18.5 us per squaring; of one set
-// 15.2 and 16.6, and 2 % more with the code of both in the kernel).
-constexpr int SMALL_BOTH = 2;
-
+// threads past a two-prime test's own only join the barriers).  A batch of
+// several sets runs in one launch: with a launch per set the second waited for
+// the first (102 tests at n = 12 of sets 0 and 1, one B200: 31.6 -> 18.5 us per
+// squaring; of one set 15.2 and 16.6, and 2 % more with the code of both in the
+// kernel).
 template <int SET, int LOGN, bool SPLIT>
-struct SmallLaunch : SmallShape<(SET == 0) ? 0 : 1, LOGN, SPLIT>
+struct SmallLaunch : SmallShape<(SET == ANY_SET) ? 1 : SET, LOGN, SPLIT>
 {
 };
 
@@ -685,9 +708,8 @@ __global__ void __launch_bounds__(SmallLaunch<SET, LOGN, SPLIT>::T, SmallLaunch<
 	const int t = a.tests[blockIdx.x];
 	if (!test_ok(a, t)) return;
 	const TestDesc &d = a.desc[t];
-	if constexpr (SET != SMALL_BOTH) small_body<SET, LOGN, SPLIT>(a, t, d, sm);
-	else if (d.set == 0) small_body<0, LOGN, SPLIT>(a, t, d, sm);
-	else small_body<1, LOGN, SPLIT>(a, t, d, sm);
+	if constexpr (SET != ANY_SET) small_body<SET, LOGN, SPLIT>(a, t, d, sm);
+	else by_set<true>(d.set, [&](auto S) { small_body<decltype(S)::value, LOGN, SPLIT>(a, t, d, sm); });
 }
 
 // ------------------------------------------------------------------ k_cluster
@@ -816,7 +838,7 @@ __device__ __forceinline__ void cluster_test(const Args &a, int t, const TestDes
 	cg::cluster_group cl = cg::this_cluster();
 	const int tid = threadIdx.x;
 	const bool owner = (tid < T0);
-	const Tables &tab = a.tab[SET];
+	const Tables &tab = a.tab[tab_of(SET)];
 	const size_t N = size_t(C) * Q;
 	const size_t nseg = N / SEG;
 
@@ -939,9 +961,9 @@ __device__ __forceinline__ void cluster_test(const Args &a, int t, const TestDes
 	if ((tid == 0) && (q == 0) && (a.dup_mode == DUP_BITS)) a.pos[t] = (pos0 - iters < -1) ? -1 : pos0 - iters;
 }
 
-// Persistent grid of clusters over the tests a.tests[0 .. ntests-1], of
-// either prime set.
-template <int LQ, int LC>
+// Persistent grid of clusters over the tests a.tests[0 .. ntests-1]: of sets 0
+// and 1 (SET = 0), all of set 3, or of any (ANY_SET).
+template <int LQ, int LC, int SET>
 __global__ void __launch_bounds__(ClusterShape<LQ, LC>::T, ClusterShape<LQ, LC>::MINB) k_cluster(const Args a, int ntests)
 {
 	pdl_wait();
@@ -957,7 +979,12 @@ __global__ void __launch_bounds__(ClusterShape<LQ, LC>::T, ClusterShape<LQ, LC>:
 		if (test_ok(a, t))
 		{
 			const TestDesc &d = a.desc[t];
-			if (d.set == 0) cluster_test<0, LQ, LC>(a, t, d, sm, q); else cluster_test<1, LQ, LC>(a, t, d, sm, q);
+			if constexpr (SET == 3) cluster_test<3, LQ, LC>(a, t, d, sm, q);
+			else if constexpr (SET == 0)
+			{
+				if (d.set == 0) cluster_test<0, LQ, LC>(a, t, d, sm, q); else cluster_test<1, LQ, LC>(a, t, d, sm, q);
+			}
+			else by_set<true>(d.set, [&](auto S_) { cluster_test<decltype(S_)::value, LQ, LC>(a, t, d, sm, q); });
 		}
 		// the next test's first shared-memory writes follow this barrier, after
 		// every CTA has read this test's last carries
@@ -1060,7 +1087,7 @@ __device__ __forceinline__ void col_fwd_body(const Args &a, const TestDesc &d, u
 		}
 	}
 	__syncthreads();
-	run_fwd<SET, LR, false, MP>(sm, S::PS, S::CWL, true, 1u, 0u, a.tab[SET]);
+	run_fwd<SET, LR, false, MP>(sm, S::PS, S::CWL, true, 1u, 0u, a.tab[tab_of(SET)]);
 	for (int e = threadIdx.x; e < S::R * S::CW / 4; e += blockDim.x)
 	{
 		const int k = e >> (S::CWL - 2), cc = (e & (S::CW / 4 - 1)) * 4;
@@ -1078,23 +1105,22 @@ __device__ __forceinline__ void col_fwd_body(const Args &a, const TestDesc &d, u
 // have returns.  The planes of a row are independent until the CRT, so a CTA
 // holds one plane (shared memory PC words) and an SM holds as many CTAs as
 // its registers allow.
-template <int SET, int LC>
+template <int SET, int LC, bool S3 = false>
 __device__ __forceinline__ void row_body(const Args &a, const TestDesc &d, uint32_t *sm)
 {
 	using S = RowShape<LC>;
-	constexpr int W = PrimeSet<SET>::W;
 	const int n = a.n, lr = n - LC;
 	const size_t N = size_t(1) << n;
 	const int P = static_cast<int>(gridDim.x >> lr);
 	const int k = static_cast<int>(blockIdx.x) / P, pl = static_cast<int>(blockIdx.x) % P;
-	if (pl >= W) return;
+	if (pl >= (((SET == 1) && S3) ? set_planes(d.set) : PrimeSet<SET>::W)) return;
 	uint32_t *buf = ((a.op == OP_FWD) ? d.zp : d.planes) + static_cast<size_t>(k) * S::C;
 	const uint32_t base = a.twist ? 1u : (1u << lr) + static_cast<uint32_t>(k);
 	using MP = RowMap<LC>;
 
 	if (a.op != OP_FWD)
 	{
-		row_core_global<SET, LC, MP>(sm, S::PC, base, a.tab[SET], d.zp + static_cast<size_t>(k) * S::C, N, a.op, buf, N,
+		row_core_global<SET, LC, MP>(sm, S::PC, base, a.tab[tab_of(SET)], d.zp + static_cast<size_t>(k) * S::C, N, a.op, buf, N,
 									 pl, pl + 1);
 		return;
 	}
@@ -1105,7 +1131,7 @@ __device__ __forceinline__ void row_body(const Args &a, const TestDesc &d, uint3
 		p[0] = u.x; p[1] = u.y; p[2] = u.z; p[3] = u.w;
 	}
 	__syncthreads();
-	run_fwd<SET, LC, false, MP>(sm, S::PC, 0, false, base, 1u, a.tab[SET], pl, pl + 1);
+	run_fwd<SET, LC, false, MP>(sm, S::PC, 0, false, base, 1u, a.tab[tab_of(SET)], pl, pl + 1);
 	for (int e = threadIdx.x; e < S::C / 4; e += blockDim.x)
 	{
 		const uint32_t *p = sm + MP::addr(4 * e, 0);
@@ -1136,7 +1162,7 @@ __device__ __forceinline__ void col_inv_body(const Args &a, const TestDesc &d, b
 		}
 	}
 	__syncthreads();
-	run_inv<SET, LR, false, MP>(sm, S::PS, S::CWL, true, 1u, 0u, a.tab[SET]);
+	run_inv<SET, LR, false, MP>(sm, S::PS, S::CWL, true, 1u, 0u, a.tab[tab_of(SET)]);
 
 	int32_t *out = d.regs + static_cast<size_t>(a.dst) * N;
 	for (int e = threadIdx.x; e < S::R * SPR; e += blockDim.x)
@@ -1171,11 +1197,11 @@ __global__ void __launch_bounds__(col_threads(LR)) k_col_fwd(const Args a)
 	bool active;
 	(void)get_dup(a, d, t, a.j, active);
 	if (!active) return;
-	if (d.set == 0) col_fwd_body<0, LR>(a, d, sm); else col_fwd_body<1, LR>(a, d, sm);
+	by_set<true>(d.set, [&](auto S) { col_fwd_body<decltype(S)::value, LR>(a, d, sm); });
 }
 
 // Rows: the last log2 C forward stages, pointwise, first inverse stages.
-template <int LC>
+template <int LC, bool S3>
 __global__ void __launch_bounds__(row_threads(LC)) k_row(const Args a)
 {
 	pdl_wait();
@@ -1186,7 +1212,7 @@ __global__ void __launch_bounds__(row_threads(LC)) k_row(const Args a)
 	(void)get_dup(a, d, t, a.j, active);
 	if (!active) return;
 	if (d.set == 0) row_body<0, LC>(a, d, sm);
-	else if (d.set == 1) row_body<1, LC>(a, d, sm);
+	else if (S3 || (d.set == 1)) row_body<1, LC, S3>(a, d, sm);
 	else row_body<2, LC>(a, d, sm);
 }
 
@@ -1260,7 +1286,7 @@ __global__ void __launch_bounds__(col_threads(LR)) k_col_inv(const Args a)
 	bool active;
 	const bool dup = get_dup(a, d, t, a.j, active);
 	if (!active) return;
-	if (d.set == 0) col_inv_body<0, LR>(a, d, dup, sm); else col_inv_body<1, LR>(a, d, dup, sm);
+	by_set<true>(d.set, [&](auto S) { col_inv_body<decltype(S)::value, LR>(a, d, dup, sm); });
 }
 
 // ---- transforms of one thread's registers.
@@ -1445,8 +1471,8 @@ __device__ __forceinline__ void mid_body(const Args &a, const TestDesc &d, uint3
 	}
 	__syncthreads();
 	const uint32_t base = (1u << MID_LR1) + static_cast<uint32_t>(m);
-	if constexpr (INV) run_inv<SET, LR2, false, MP>(sm, S::PS, S::CWL, true, base, 0u, a.tab[SET]);
-	else run_fwd<SET, LR2, false, MP>(sm, S::PS, S::CWL, true, base, 0u, a.tab[SET]);
+	if constexpr (INV) run_inv<SET, LR2, false, MP>(sm, S::PS, S::CWL, true, base, 0u, a.tab[tab_of(SET)]);
+	else run_fwd<SET, LR2, false, MP>(sm, S::PS, S::CWL, true, base, 0u, a.tab[tab_of(SET)]);
 	for (int e = threadIdx.x; e < S::R * S::CW / 4; e += blockDim.x)
 	{
 		const int k = e >> (S::CWL - 2), cc = (e & (S::CW / 4 - 1)) * 4;
@@ -1467,9 +1493,8 @@ __global__ void __launch_bounds__(col_threads(LR2)) k_mid(const Args a)
 	bool active;
 	(void)get_dup(a, d, t, a.j, active);
 	if (!active) return;
-	if (d.set == 0) mid_body<0, LR2, INV>(a, d, sm);
-	else if (d.set == 1) mid_body<1, LR2, INV>(a, d, sm);
-	else mid_body<2, LR2, INV>(a, d, sm);
+	if (d.set == 2) mid_body<2, LR2, INV>(a, d, sm);
+	else by_set<true>(d.set, [&](auto S) { mid_body<decltype(S)::value, LR2, INV>(a, d, sm); });
 }
 
 // The middle pass in registers: a thread owns one column of one plane of one
@@ -1481,10 +1506,10 @@ __global__ void __launch_bounds__(col_threads(LR2)) k_mid(const Args a)
 constexpr int MIDR_THREADS = 128;
 constexpr int MIDR_LOG = 7;
 
-template <int SET, int LR2, bool INV>
+template <int SET, int LR2, bool INV, bool S3 = false>
 __device__ __forceinline__ void midr_body(const Args &a, const TestDesc &d, int m, int pl, size_t c)
 {
-	if (pl >= PrimeSet<SET>::W) return;
+	if (pl >= (((SET == 1) && S3) ? set_planes(d.set) : PrimeSet<SET>::W)) return;
 	const int lc = a.n - MID_LR1 - LR2;
 	const size_t N = size_t(1) << a.n, C = size_t(1) << lc;
 	uint32_t *p = ((a.op == OP_FWD) ? d.zp : d.planes) + static_cast<size_t>(pl) * N +
@@ -1499,17 +1524,17 @@ __device__ __forceinline__ void midr_body(const Args &a, const TestDesc &d, int 
 	{
 		if (a.twist)
 		{
-			const uint32_t *tt = a.tab[SET].ti[pl];
+			const uint32_t *tt = a.tab[tab_of(SET)].ti[pl];
 			twist_regs<Z, LR2>(z, x, twist_start(tt, m, c, C), twist_step<Z>(tt, c, C));
 		}
-		inv_thread<Z, LR2>(z, x, base, a.tab[SET].iv[pl]);
+		inv_thread<Z, LR2>(z, x, base, a.tab[tab_of(SET)].iv[pl]);
 	}
 	else
 	{
-		fwd_thread<Z, LR2>(z, x, base, a.tab[SET].fw[pl]);
+		fwd_thread<Z, LR2>(z, x, base, a.tab[tab_of(SET)].fw[pl]);
 		if (a.twist)
 		{
-			const uint32_t *tt = a.tab[SET].tf[pl];
+			const uint32_t *tt = a.tab[tab_of(SET)].tf[pl];
 			twist_regs<Z, LR2>(z, x, twist_start(tt, m, c, C), twist_step<Z>(tt, c, C));
 		}
 	}
@@ -1520,7 +1545,7 @@ __device__ __forceinline__ void midr_body(const Args &a, const TestDesc &d, int 
 // 32-word columns (lr2 = 5) fit four CTAs per SM in 128 registers.
 __host__ __device__ constexpr int midr_min_blocks(int lr2) { return (lr2 == 5) ? 4 : 1; }
 
-template <int LR2, bool INV>
+template <int LR2, bool INV, bool S3>
 __global__ void __launch_bounds__(MIDR_THREADS, midr_min_blocks(LR2)) k_midr(const Args a)
 {
 	pdl_wait();
@@ -1535,7 +1560,7 @@ __global__ void __launch_bounds__(MIDR_THREADS, midr_min_blocks(LR2)) k_midr(con
 	const int m = q / P, pl = q % P;
 	const size_t c = (static_cast<size_t>(blockIdx.x & ((1u << chunks_log) - 1)) << MIDR_LOG) + threadIdx.x;
 	if (d.set == 0) midr_body<0, LR2, INV>(a, d, m, pl, c);
-	else if (d.set == 1) midr_body<1, LR2, INV>(a, d, m, pl, c);
+	else if (S3 || (d.set == 1)) midr_body<1, LR2, INV, S3>(a, d, m, pl, c);
 	else midr_body<2, LR2, INV>(a, d, m, pl, c);
 }
 
@@ -1554,10 +1579,10 @@ constexpr int MIDP_THREADS = 128;
 constexpr int MIDP_COLS = MIDP_THREADS / 2;
 constexpr int MIDP_COLS_LOG = 6;
 
-template <int SET, bool INV>
+template <int SET, bool INV, bool S3 = false>
 __device__ __forceinline__ void midp_body(const Args &a, const TestDesc &d, int m, int pl, size_t c, int h)
 {
-	if (pl >= PrimeSet<SET>::W) return;
+	if (pl >= (((SET == 1) && S3) ? set_planes(d.set) : PrimeSet<SET>::W)) return;
 	constexpr int LR2 = 6;
 	const int lc = a.n - MID_LR1 - LR2;
 	const size_t N = size_t(1) << a.n, C = size_t(1) << lc;
@@ -1576,7 +1601,7 @@ __device__ __forceinline__ void midp_body(const Args &a, const TestDesc &d, int 
 			x[16 + i] = p[static_cast<size_t>(32 + 16 * h + i) * C];
 		}
 		typename Z::root_t w0[1];
-		load_twiddles<1>(w0, base, a.tab[SET].fw[pl]);
+		load_twiddles<1>(w0, base, a.tab[tab_of(SET)].fw[pl]);
 #pragma unroll
 		for (int i = 0; i < 16; ++i) bfly_ct(z, x[i], x[16 + i], w0[0]);
 		// h = 0 keeps rows 0..15 and takes 16..31; h = 1 keeps 48..63 and takes 32..47
@@ -1587,7 +1612,7 @@ __device__ __forceinline__ void midp_body(const Args &a, const TestDesc &d, int 
 			const uint32_t recv = __shfl_xor_sync(0xffffffffu, send, 1);
 			if (h) x[i] = recv; else x[16 + i] = recv;
 		}
-		fwd_thread<Z, 5>(z, x, 2u * base + static_cast<uint32_t>(h), a.tab[SET].fw[pl]);
+		fwd_thread<Z, 5>(z, x, 2u * base + static_cast<uint32_t>(h), a.tab[tab_of(SET)].fw[pl]);
 #pragma unroll
 		for (int i = 0; i < 32; ++i) p[static_cast<size_t>(32 * h + i) * C] = x[i];
 	}
@@ -1595,7 +1620,7 @@ __device__ __forceinline__ void midp_body(const Args &a, const TestDesc &d, int 
 	{
 #pragma unroll
 		for (int i = 0; i < 32; ++i) x[i] = p[static_cast<size_t>(32 * h + i) * C];
-		inv_thread<Z, 5>(z, x, 2u * base + static_cast<uint32_t>(h), a.tab[SET].iv[pl]);
+		inv_thread<Z, 5>(z, x, 2u * base + static_cast<uint32_t>(h), a.tab[tab_of(SET)].iv[pl]);
 		// back to the pairs of the first stage: h = 0 holds rows 0..15 with
 		// 32..47, h = 1 rows 16..31 with 48..63
 #pragma unroll
@@ -1606,7 +1631,7 @@ __device__ __forceinline__ void midp_body(const Args &a, const TestDesc &d, int 
 			if (h) x[i] = recv; else x[16 + i] = recv;
 		}
 		typename Z::root_t w0[1];
-		load_twiddles<1>(w0, base, a.tab[SET].iv[pl]);
+		load_twiddles<1>(w0, base, a.tab[tab_of(SET)].iv[pl]);
 #pragma unroll
 		for (int i = 0; i < 16; ++i) bfly_gs(z, x[i], x[16 + i], w0[0]);
 #pragma unroll
@@ -1618,7 +1643,7 @@ __device__ __forceinline__ void midp_body(const Args &a, const TestDesc &d, int 
 	}
 }
 
-template <bool INV>
+template <bool INV, bool S3>
 __global__ void __launch_bounds__(MIDP_THREADS, 4) k_midp(const Args a)
 {
 	pdl_wait();
@@ -1634,7 +1659,7 @@ __global__ void __launch_bounds__(MIDP_THREADS, 4) k_midp(const Args a)
 	const int h = static_cast<int>(threadIdx.x & 1);
 	const size_t c = (static_cast<size_t>(blockIdx.x & ((1u << chunks_log) - 1)) << MIDP_COLS_LOG) + (threadIdx.x >> 1);
 	if (d.set == 0) midp_body<0, INV>(a, d, m, pl, c, h);
-	else if (d.set == 1) midp_body<1, INV>(a, d, m, pl, c, h);
+	else if (S3 || (d.set == 1)) midp_body<1, INV, S3>(a, d, m, pl, c, h);
 	else midp_body<2, INV>(a, d, m, pl, c, h);
 }
 
@@ -1683,7 +1708,7 @@ __device__ __forceinline__ void col_fwd_reg_body(const Args &a, const TestDesc &
 		uint32_t x[R];
 #pragma unroll
 		for (int k = 0; k < R; ++k) x[k] = Z::from_int(dv[k]);
-		fwd_reg<Z, LR>(Z{}, x, 1u, a.tab[SET].fw[PL]);
+		fwd_reg<Z, LR>(Z{}, x, 1u, a.tab[tab_of(SET)].fw[PL]);
 #pragma unroll
 		for (int k = 0; k < R; ++k) dst[PL * N + k * C] = x[k];
 	});
@@ -1709,7 +1734,7 @@ __device__ __forceinline__ void col_inv_reg_body(const Args &a, const TestDesc &
 		uint32_t x[R];
 #pragma unroll
 		for (int k = 0; k < R; ++k) x[k] = src[k * C];
-		inv_reg<Z, LR>(Z{}, x, 1u, a.tab[SET].iv[PL], true, __ldg(&a.tab[SET].fw[PL][0]), __ldg(&a.tab[SET].iv[PL][0]));
+		inv_reg<Z, LR>(Z{}, x, 1u, a.tab[tab_of(SET)].iv[PL], true, __ldg(&a.tab[tab_of(SET)].fw[PL][0]), __ldg(&a.tab[tab_of(SET)].iv[PL][0]));
 #pragma unroll
 		for (int k = 0; k < R; ++k) sm[PL * PS + MP::addr(k, tid)] = x[k];
 	});
@@ -1737,7 +1762,7 @@ __device__ __forceinline__ void col_inv_reg_body(const Args &a, const TestDesc &
 }
 
 // Shared memory: [R][T + T/16] int32 staging of the digits when fixing carries.
-template <int LR>
+template <int LR, bool S3>
 __global__ void __launch_bounds__(COLR_THREADS) k_colr_fwd(const Args a)
 {
 	pdl_wait();
@@ -1747,7 +1772,7 @@ __global__ void __launch_bounds__(COLR_THREADS) k_colr_fwd(const Args a)
 	bool active;
 	(void)get_dup(a, d, t, a.j, active);
 	if (!active) return;
-	if (d.set == 0) col_fwd_reg_body<0, LR>(a, d, sm); else col_fwd_reg_body<1, LR>(a, d, sm);
+	by_set<S3>(d.set, [&](auto S) { col_fwd_reg_body<decltype(S)::value, LR>(a, d, sm); });
 }
 
 template <int LR>
@@ -1756,7 +1781,7 @@ struct ColRegShape
 	static constexpr size_t SMEM = size_t(WMAX) * (1 << LR) * (COLR_THREADS + COLR_THREADS / 16) * 4;
 };
 
-template <int LR>
+template <int LR, bool S3>
 __global__ void __launch_bounds__(COLR_THREADS) k_colr_inv(const Args a)
 {
 	pdl_wait();
@@ -1766,7 +1791,7 @@ __global__ void __launch_bounds__(COLR_THREADS) k_colr_inv(const Args a)
 	bool active;
 	const bool dup = get_dup(a, d, t, a.j, active);
 	if (!active) return;
-	if (d.set == 0) col_inv_reg_body<0, LR>(a, d, dup, sm); else col_inv_reg_body<1, LR>(a, d, dup, sm);
+	by_set<S3>(d.set, [&](auto S) { col_inv_reg_body<decltype(S)::value, LR>(a, d, dup, sm); });
 }
 
 // ---- plane-split register columns, for batches too small to fill the GPU
@@ -1809,7 +1834,7 @@ __device__ __forceinline__ void col_fwd_split_body(const Args &a, const TestDesc
 #pragma unroll
 	for (int k = 0; k < R; ++k)
 		x[k] = z.from_int(a.fix ? sm[k * RW + c + c / SEG] : srcreg[static_cast<size_t>(k) * C + c0 + c]);
-	fwd_reg<decltype(z), LR>(z, x, 1u, a.tab[SET].fw[pl]);
+	fwd_reg<decltype(z), LR>(z, x, 1u, a.tab[tab_of(SET)].fw[pl]);
 	uint32_t *dst = ((a.op == OP_FWD) ? d.zp : d.planes) + pl * N + c0 + c;
 #pragma unroll
 	for (int k = 0; k < R; ++k) dst[k * C] = x[k];
@@ -1831,8 +1856,8 @@ __device__ __forceinline__ void col_inv_split_body(const Args &a, const TestDesc
 		uint32_t x[R];
 #pragma unroll
 		for (int k = 0; k < R; ++k) x[k] = src[k * C];
-		inv_reg<decltype(z), LR>(z, x, 1u, a.tab[SET].iv[pl], true, __ldg(&a.tab[SET].fw[pl][0]),
-								 __ldg(&a.tab[SET].iv[pl][0]));
+		inv_reg<decltype(z), LR>(z, x, 1u, a.tab[tab_of(SET)].iv[pl], true, __ldg(&a.tab[tab_of(SET)].fw[pl][0]),
+								 __ldg(&a.tab[tab_of(SET)].iv[pl][0]));
 #pragma unroll
 		for (int k = 0; k < R; ++k) sm[pl * PS + MP::addr(k, c)] = x[k];
 	}
@@ -1859,7 +1884,7 @@ __device__ __forceinline__ void col_inv_split_body(const Args &a, const TestDesc
 	}
 }
 
-template <int LR>
+template <int LR, bool S3>
 __global__ void __launch_bounds__(WMAX * CS_T) k_colr_fwd_s(const Args a)
 {
 	pdl_wait();
@@ -1869,10 +1894,10 @@ __global__ void __launch_bounds__(WMAX * CS_T) k_colr_fwd_s(const Args a)
 	bool active;
 	(void)get_dup(a, d, t, a.j, active);
 	if (!active) return;
-	if (d.set == 0) col_fwd_split_body<0, LR>(a, d, sm); else col_fwd_split_body<1, LR>(a, d, sm);
+	by_set<S3>(d.set, [&](auto S) { col_fwd_split_body<decltype(S)::value, LR>(a, d, sm); });
 }
 
-template <int LR>
+template <int LR, bool S3>
 __global__ void __launch_bounds__(WMAX * CS_T) k_colr_inv_s(const Args a)
 {
 	pdl_wait();
@@ -1882,7 +1907,7 @@ __global__ void __launch_bounds__(WMAX * CS_T) k_colr_inv_s(const Args a)
 	bool active;
 	const bool dup = get_dup(a, d, t, a.j, active);
 	if (!active) return;
-	if (d.set == 0) col_inv_split_body<0, LR>(a, d, dup, sm); else col_inv_split_body<1, LR>(a, d, dup, sm);
+	by_set<S3>(d.set, [&](auto S) { col_inv_split_body<decltype(S)::value, LR>(a, d, dup, sm); });
 }
 
 // ---- packed digits (prime set 2).
@@ -2257,6 +2282,8 @@ __global__ void __launch_bounds__(4 * PCS_T, MINB) k_pcol_inv_s(const Args a)
 	pcol_inv_split_body<LR>(a, d, dup, sm);
 }
 
+#ifndef GFC_TEMPLATES_ONLY      // the kernels that are no templates: in gf_host.cu only
+
 // Pending packed carries of register a.dst absorbed (a.n = n: digits).
 __global__ void __launch_bounds__(256) k_pfixup(const Args a)
 {
@@ -2510,5 +2537,7 @@ __global__ void k_pos_sub(int64_t *pos, const int32_t *tests, int ntests, int co
 		pos[tests[i]] = (p < -1) ? -1 : p;
 	}
 }
+
+#endif
 
 }  // namespace gfc

@@ -9,7 +9,7 @@ the GPU tests):
   mixed-radix digits decides V > M/2, and with the top digit a4 - p4 when it
   does, f V = sum_{j<5} U_j b^j for the base-b limbs of f p1, f p1 p2,
   f p1 p2 p3, with |U_j| and every window position inside the stated bounds;
-* the fused CRT + carry of prime sets 0 and 1 (crt_carry<SET>): one 64-bit
+* the fused CRT + carry of prime sets 0, 1 and 3 (crt_carry<SET>): one 64-bit
   division by b and per-test constants give the balanced digit and the carry
   of f V + c exactly;
 * the absorption of a segment's carry into the next 16 digits (absorb,
@@ -133,7 +133,7 @@ def test_window_bounds(b):
     assert math.log2(2**max(even, odd) + 2**carry) < 61.4 < 62
 
 
-# ---- the fused CRT + carry of prime sets 0 and 1 (gf_arith.cuh crt_carry<SET>)
+# ---- the fused CRT + carry of prime sets 0, 1 and 3 (gf_arith.cuh crt_carry<SET>)
 
 P0 = (125 * 2**25 + 1, 243 * 2**24 + 1)
 MASK = 2**64 - 1
@@ -180,7 +180,7 @@ def crt_carry(x, dup, K, c, primes):
     return rv - K["h"], cout
 
 
-@pytest.mark.parametrize("primes", [P0, P31], ids=["set0", "set1"])
+@pytest.mark.parametrize("primes", [P0, P31, P31[:2]], ids=["set0", "set1", "set3"])
 @pytest.mark.parametrize("b", [8, 1_000, 65_538, 22_000_000, 1_000_000_000, 2**31 - 2])
 def test_fused_crt_carry_is_exact(primes, b):
     """digit + b * carry_out = f V_c + carry_in with the digit in [-b/2, b - b/2)
