@@ -26,6 +26,7 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC,-fvisibility=hidden",
     "-shared",
     "--threads", "0",       # the sources in parallel
+    "-static-global-template-stub=false",   # kernel templates instantiated in one file, launched from another
 ]
 
 

@@ -1352,8 +1352,8 @@ void op_square_mul(gfc_batch &bt, int32_t m)
 	a.dst = 0;
 	const unsigned nseg = static_cast<unsigned>(bt.N / SEG);
 	const dim3 grid((nseg + FIX_THREADS - 1) / FIX_THREADS, static_cast<unsigned>(bt.count));
-	k_mulscalar<<<grid, FIX_THREADS, 0, bt.stream>>>(a, m);
-	after_launch();
+	a.count = m;
+	launch_pdl(k_mulscalar, grid, dim3(FIX_THREADS), 0, bt.stream, a);
 	bt.pending = 0;
 }
 

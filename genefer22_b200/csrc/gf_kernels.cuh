@@ -2345,10 +2345,10 @@ __global__ void __launch_bounds__(256) k_fixup(const Args a)
 	for (int i = 0; i < SEG / 4; ++i) p[i] = make_int4(dg[4 * i], dg[4 * i + 1], dg[4 * i + 2], dg[4 * i + 3]);
 }
 
-// r_dst = m r_dst digit by digit, carrying inside 16-digit segments and leaving
+// r_dst = m r_dst (m = a.count) digit by digit, carrying inside 16-digit segments and leaving
 // the segment carries for k_fixup: the digit-times-scalar step of
 // transform::squareMul (src/transformCPUi32.h:774-797).  |digit m| < 2^62.
-__global__ void __launch_bounds__(256) k_mulscalar(const Args a, int32_t m)
+__global__ void __launch_bounds__(256) k_mulscalar(const Args a)
 {
 	pdl_wait();
 	const int t = a.tests[blockIdx.y];
@@ -2367,7 +2367,7 @@ __global__ void __launch_bounds__(256) k_mulscalar(const Args a, int32_t m)
 	}
 	int64_t c = 0;
 #pragma unroll
-	for (int i = 0; i < SEG; ++i) dg[i] = carry_wide(static_cast<int64_t>(dg[i]) * m + c, d.ck, c);
+	for (int i = 0; i < SEG; ++i) dg[i] = carry_wide(static_cast<int64_t>(dg[i]) * a.count + c, d.ck, c);
 #pragma unroll
 	for (int i = 0; i < SEG / 4; ++i) p[i] = make_int4(dg[4 * i], dg[4 * i + 1], dg[4 * i + 2], dg[4 * i + 3]);
 	d.carry[s] = c;
