@@ -103,9 +103,8 @@ __device__ __forceinline__ void for_planes(F &&f)
 // Kernels of unpacked launches come with and without S3: a batch none of whose
 // tests was on set 3 when it was made keeps its tests on sets 0 and 1, and its
 // kernels hold the bodies of those only.  (With the third body in every kernel
-// ptxas took more registers or another schedule: one B200, 3-prime batches of 64
-// at n = 16 125.3 -> 127.5 us per squaring, at n = 15 66.8 -> 68.7, a lone packed
-// test at n = 20 43.0 -> 44.4.)  Set 3 runs set 1's row and middle passes on its
+// ptxas takes more registers or another schedule: three-prime batches of 64 at
+// n = 15, 16 measured 1.5-3 % slower on one B200, and equal in this form.)  Set 3 runs set 1's row and middle passes on its
 // first two planes.
 constexpr int ANY_SET = 4;       // template argument of kernels that take each test's set as it comes
 
