@@ -1302,6 +1302,19 @@ void fourstep(gfc_batch &bt, Args a)
 	bt.pending = a.dst;
 }
 
+// Whether the cluster kernel can absorb the carries pending on register 0
+// when it loads the tests.  The owners of its short rows (n <= 14) hold 8
+// digits, and up to n = 14 the only pending carries are squareMul's, of
+// magnitude at most 2^31 (b/2 + 1) / (b - 1) < 2^31: seven digits bring those
+// to one unit where b^7 >= 2^31, from b = 22.  Below, the stand-alone fix-up
+// spreads them over the segment's 16 digits.
+bool cluster_absorbs(const gfc_batch &bt)
+{
+	if (bt.n > SMALL_MAX_LOGN) return true;
+	for (uint32_t b : bt.b) if (b < 22) return false;
+	return true;
+}
+
 // count squarings of r_0 (dup_mode DUP_NONE / DUP_ALL / DUP_BITS).
 void op_square(gfc_batch &bt, int dup_mode, uint32_t count)
 {
@@ -1310,7 +1323,7 @@ void op_square(gfc_batch &bt, int dup_mode, uint32_t count)
 	{
 		// digits stay in shared memory for all `count` squarings; carries
 		// pending on register 0 are absorbed when a test is loaded
-		if ((bt.pending >= 0) && (bt.pending != 0)) materialize(bt);
+		if ((bt.pending >= 0) && ((bt.pending != 0) || !cluster_absorbs(bt))) materialize(bt);
 		Args a = make_args(bt);
 		a.op = OP_SQUARE; a.dup_mode = dup_mode; a.src = 0; a.dst = 0;
 		a.count = static_cast<int>(count);
@@ -1383,7 +1396,7 @@ void op_mul(gfc_batch &bt, size_t dst)
 void time_kernels(gfc_batch &bt, uint32_t reps, float *ms)
 {
 	no_capture(bt);
-	if ((bt.pending >= 0) && (bt.pending != 0)) materialize(bt);
+	if ((bt.pending >= 0) && ((bt.pending != 0) || ((bt.cluster > 0) && !cluster_absorbs(bt)))) materialize(bt);
 	cudaEvent_t ev[5];
 	for (auto &e : ev) GFC_CK(cudaEventCreate(&e));
 	double acc[5] = { 0, 0, 0, 0, 0 };

@@ -741,9 +741,10 @@ struct ClusterShape
 	static constexpr int PC = C + C / 32;                 // padded plane (RowMap)
 	static constexpr bool PS = (LC <= 11);                // plane-split passes
 	// digits per owner thread: 16 (one carry segment of the engine), or 8 for
-	// the short rows, whose owners then run half as long a carry chain (the
-	// carries inside the kernel are its own; every carry fits 8 digits for
-	// b >= 1024, absorb() checks it)
+	// the short rows, whose owners then run half as long a carry chain.  The
+	// carries inside the kernel are its own, at most 2 N (b/2 + 1)^2 / (b - 1),
+	// below b^7 for every b >= 8 at n <= 14; carries pending when a test is
+	// loaded fit where the host says so (cluster_absorbs); absorb() checks both
 	static constexpr int D = PS ? SEG / 2 : SEG;
 	static constexpr int T0 = C / D;                      // owner threads
 	static constexpr int T = PS ? WMAX * C / 8 : T0;

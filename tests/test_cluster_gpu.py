@@ -117,3 +117,22 @@ def test_cluster_finished_test_sits_out(oracle):
         for k in range(j.nbits - 1, -1, -1):
             o.squareDup(bool((e >> k) & 1))
         assert np.array_equal(canon(bt.get(i, 0), j.b), canon(o.getInt(), j.b)), i
+
+
+@pytest.mark.parametrize("n", [12, 13, 14])
+@pytest.mark.parametrize("b", [8, 16, 20, 22, 1024])
+def test_square_mul_carry_into_the_next_squaring(oracle, n, b):
+    """squareMul by a large a leaves segment carries of up to 2^31 pending, which
+    the next squaring absorbs: more than 8 digits of a base below 22 hold."""
+    t = Transform(b, n)
+    assert t.batch.plan() == PLAN_CLUSTER
+    o = oracle.OracleTransform(b, n)
+    d = rand_digits(np.random.default_rng(b * n), b, 1 << n)
+    t.setInt(d)
+    o.setInt(d)
+    for a in (0x7fffffff, -0x7fffffff):
+        t.squareMul(a); o.squareMul(a)
+        t.squareDup(True); o.squareDup(True)
+        t.squareMul(a); o.squareMul(a)
+        t.squareMul(3); o.squareMul(3)
+        assert np.array_equal(canon(t.getInt(), b), canon(o.getInt(), b)), a
