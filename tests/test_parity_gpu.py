@@ -257,6 +257,20 @@ def test_square_mul(oracle, b, plan):
         assert np.array_equal(canon(g, b), canon(o.getInt(), b)), f"a={a}"
 
 
+@pytest.mark.parametrize("plan", [0, 1, 3])
+def test_time_kernels_squares_the_register_as_it_stands(oracle, plan):
+    """gfc_batch_time_kernels squares register 0, also where squareMul has left carries pending."""
+    b, n = 1_000_002, 12
+    t, o = Transform(b, n), oracle.OracleTransform(b, n)
+    t.batch.set_plan(plan)
+    d = rand_digits(np.random.default_rng(plan), b, 1 << n)
+    t.setInt(d); o.setInt(d)
+    t.squareMul(12345); o.squareMul(12345)
+    t.batch.time_kernels(2)
+    o.squareDup(False); o.squareDup(False)
+    assert np.array_equal(canon(t.getInt(), b), canon(o.getInt(), b))
+
+
 @pytest.mark.parametrize("b", [10, 1026, LARGE_B])
 def test_digit_range_checked_on_load(b):
     """gfc_batch_set_zi / gfc_batch_set_all accept |d| <= b/2 + 1 and refuse one
