@@ -2147,6 +2147,7 @@ GFC_API int gfc_batch_assign(gfc_batch *bt, size_t test, uint32_t b)
 		if ((b < 8) || (b >= (1u << 31))) fail(GFC_ERR_ARG, "assign: base b must satisfy 8 <= b < 2^31");
 		const int s = choose_set(b, bt->n, bt->s3);
 		if (s < 0) fail(GFC_ERR_RANGE, "assign: (b, n) is outside the exact range of the RNS prime sets");
+		if (bt->packed && !packed_ok(b, bt->n)) fail(GFC_ERR_RANGE, "assign: base outside the range of packed digits");
 		cudaSetDevice(bt->device);
 		materialize(*bt);
 		GFC_CK(cudaStreamSynchronize(bt->stream));
@@ -2155,7 +2156,6 @@ GFC_API int gfc_batch_assign(gfc_batch *bt, size_t test, uint32_t b)
 		bt->b[test] = b;
 		bt->set[test] = s;
 		bt->nset[s]++;
-		if (bt->packed && !packed_ok(b, bt->n)) fail(GFC_ERR_RANGE, "assign: base outside the range of packed digits");
 		TestDesc &d = bt->h_desc[test];
 		d.b = b;
 		d.set = s;

@@ -98,6 +98,25 @@ def test_range_refused():
         bt.assign(0, B_MAX[16] + 2)
 
 
+def test_refused_assign_changes_nothing(oracle):
+    """The slot of a refused assign keeps its base, also for a later change of plan."""
+    n, b = 16, 2_000_002
+    bt, o = Batch([b], n), oracle.OracleTransform(b, n)
+    with pytest.raises(GfcError):
+        bt.assign(0, B_MAX[n] + 2)
+    d = rand_digits(np.random.default_rng(n), b, 1 << n)
+    bad = d.copy()
+    bad[3] = b                                # a digit of the refused base
+    with pytest.raises(GfcError):
+        bt.put(0, bad)
+    bt.put(0, d); o.setInt(d)
+    for plan in (203, 4):
+        bt.set_plan(plan)
+        bt.square(True, 1); o.squareDup(True)
+        assert np.array_equal(canon(bt.get(0), b), canon(o.getInt(), b)), plan
+    assert list(bt.widths()) == [2]
+
+
 def _blocks(bases, n, plan, B, nblk, exps):
     bt = Batch(bases, n)
     bt.set_plan(plan)
