@@ -557,11 +557,11 @@ int sm_count()
 	return v;
 }
 
-template <int SET, int LOGN>
+template <int SETS, int LOGN>
 void small_t(const Args &a, int grid, cudaStream_t s, bool prep)
 {
 	// n = 10, 11 have the kernel of any set only
-	constexpr int ST = (LOGN >= 12) ? SET : ANY_SET;
+	constexpr int ST = (LOGN >= 12) ? SETS : SETS_ANY;
 	using L = SmallLaunch<ST, LOGN, false>;
 	using LS = SmallLaunch<ST, LOGN, true>;
 	if (prep) set_smem(k_small<ST, LOGN, false>, L::SMEM);
@@ -574,16 +574,16 @@ void small_t(const Args &a, int grid, cudaStream_t s, bool prep)
 	if (!prep) launch_pdl(k_small<ST, LOGN, false>, dim3(grid), dim3(L::T), L::SMEM, s, a);
 }
 
-template <int SET>
+template <int SETS>
 void small_set(int logn, const Args &a, int grid, cudaStream_t s, bool prep)
 {
 	switch (logn)
 	{
-		case 10: small_t<SET, 10>(a, grid, s, prep); break;
-		case 11: small_t<SET, 11>(a, grid, s, prep); break;
-		case 12: small_t<SET, 12>(a, grid, s, prep); break;
-		case 13: small_t<SET, 13>(a, grid, s, prep); break;
-		case 14: small_t<SET, 14>(a, grid, s, prep); break;
+		case 10: small_t<SETS, 10>(a, grid, s, prep); break;
+		case 11: small_t<SETS, 11>(a, grid, s, prep); break;
+		case 12: small_t<SETS, 12>(a, grid, s, prep); break;
+		case 13: small_t<SETS, 13>(a, grid, s, prep); break;
+		case 14: small_t<SETS, 14>(a, grid, s, prep); break;
 		default: fail(GFC_ERR_ARG, "single-CTA plan needs 10 <= n <= 14");
 	}
 }
@@ -752,11 +752,11 @@ void launch_pcol(int lr, bool inv, const Args &a, int grid_y, cudaStream_t s, bo
 // allows 16-CTA clusters and returns in *max_out how many clusters fit on the
 // device at once; otherwise launches a persistent grid of
 // min(ntests, max_active) clusters over the tests a.tests[0 .. ntests-1].
-template <int LQ, int LC, int SET>
+template <int LQ, int LC, int SETS>
 void cluster_set(const Args &a, int ntests, int max_active, cudaStream_t s, bool prep, int *max_out)
 {
 	using S = ClusterShape<LQ, LC>;
-	auto kern = k_cluster<LQ, LC, SET>;
+	auto kern = k_cluster<LQ, LC, SETS>;
 	cudaLaunchConfig_t cfg = {};
 	cudaLaunchAttribute at[1];
 	at[0].id = cudaLaunchAttributeClusterDimension;
@@ -791,14 +791,17 @@ void cluster_set(const Args &a, int ntests, int max_active, cudaStream_t s, bool
 	after_launch();
 }
 
-// `set`: 0 (sets 0 and 1), 3 (set 3 only; n = 12..14), or ANY_SET.
+// `sets`: the kernel's, one of SETS_01, SETS_ANY and (n <= 14) SETS_3, SETS_03.
 template <int LQ, int LC>
-void cluster_t(const Args &a, int ntests, int max_active, int set, cudaStream_t s, bool prep, int *max_out)
+void cluster_t(const Args &a, int ntests, int max_active, int sets, cudaStream_t s, bool prep, int *max_out)
 {
-	if (prep || (set == 0)) cluster_set<LQ, LC, 0>(a, ntests, max_active, s, prep, max_out);
+	if (prep || (sets == SETS_01)) cluster_set<LQ, LC, SETS_01>(a, ntests, max_active, s, prep, max_out);
 	if constexpr (LC <= 10)
-		if (prep || (set == 3)) cluster_set<LQ, LC, 3>(a, ntests, max_active, s, prep, max_out);
-	if (prep || (set == ANY_SET)) cluster_set<LQ, LC, ANY_SET>(a, ntests, max_active, s, prep, max_out);
+	{
+		if (prep || (sets == SETS_3)) cluster_set<LQ, LC, SETS_3>(a, ntests, max_active, s, prep, max_out);
+		if (prep || (sets == SETS_03)) cluster_set<LQ, LC, SETS_03>(a, ntests, max_active, s, prep, max_out);
+	}
+	if (prep || (sets == SETS_ANY)) cluster_set<LQ, LC, SETS_ANY>(a, ntests, max_active, s, prep, max_out);
 }
 
 // Cluster shape by size: n = 12..14 with plane-split passes on rows of
@@ -807,17 +810,17 @@ void cluster_t(const Args &a, int ntests, int max_active, int set, cudaStream_t 
 // 8 -> 16 CTAs with the balanced row schedule: n = 12 6.75 -> 9.95 (2^8-point
 // rows of two 16-point passes leave half of the threads idle), n = 13 8.80 ->
 // 8.31; n = 14 13.04 (eight CTAs, earlier schedule) -> 10.40.
-void launch_cluster_n(int n, const Args &a, int ntests, int max_active, int set, cudaStream_t s, bool prep, int *max_out)
+void launch_cluster_n(int n, const Args &a, int ntests, int max_active, int sets, cudaStream_t s, bool prep, int *max_out)
 {
 	if (prep) *max_out = 1 << 30;
 	switch (n)
 	{
-		case 12: cluster_t<3, 9>(a, ntests, max_active, set, s, prep, max_out); break;
-		case 13: cluster_t<4, 9>(a, ntests, max_active, set, s, prep, max_out); break;
-		case 14: cluster_t<4, 10>(a, ntests, max_active, set, s, prep, max_out); break;
-		case 15: cluster_t<2, 13>(a, ntests, max_active, set, s, prep, max_out); break;
-		case 16: cluster_t<3, 13>(a, ntests, max_active, set, s, prep, max_out); break;
-		case 17: cluster_t<4, 13>(a, ntests, max_active, set, s, prep, max_out); break;
+		case 12: cluster_t<3, 9>(a, ntests, max_active, sets, s, prep, max_out); break;
+		case 13: cluster_t<4, 9>(a, ntests, max_active, sets, s, prep, max_out); break;
+		case 14: cluster_t<4, 10>(a, ntests, max_active, sets, s, prep, max_out); break;
+		case 15: cluster_t<2, 13>(a, ntests, max_active, sets, s, prep, max_out); break;
+		case 16: cluster_t<3, 13>(a, ntests, max_active, sets, s, prep, max_out); break;
+		case 17: cluster_t<4, 13>(a, ntests, max_active, sets, s, prep, max_out); break;
 		default: fail(GFC_ERR_ARG, "cluster plan needs 12 <= n <= 17");
 	}
 }
@@ -988,7 +991,7 @@ struct gfc_batch
 	std::vector<uint32_t *> ebits;
 	int nset[4] = { 0, 0, 0, 0 }; // tests per prime set (0, 1, 3)
 	int pending = -1;             // register whose segment carries are not yet absorbed (four-step)
-	uint64_t sets_version = 0;    // bumped when a test changes prime set (the single-CTA kernel is chosen by the sets present)
+	uint64_t widths_version = 0;  // bumped when a test changes its number of primes (launch_sets)
 	int cluster = 0;              // 1 when squarings use k_cluster (shape by n), else 0
 	int six = 0;                  // lr2 of a six-step plan (columns 2^4 x 2^lr2, lr = 4 + lr2), else 0
 	bool packed = false;          // prime set 2, two digits per coefficient, transform of N/2 (lr of that)
@@ -1030,8 +1033,8 @@ struct gfc_graph
 	cudaGraph_t graph = nullptr;
 	cudaGraphExec_t exec = nullptr;
 	uint64_t kernels = 0;         // kernel nodes recorded
-	uint64_t sets_version = 0;    // batch's sets_version at capture
-	bool per_set = false;         // recorded the kernel of the prime sets present (single-CTA plan)
+	uint64_t widths_version = 0;  // batch's widths_version at capture
+	bool per_width = false;       // recorded kernels of the numbers of primes present (launch_sets)
 	~gfc_graph()
 	{
 		cudaSetDevice(device);
@@ -1140,41 +1143,40 @@ Args make_args(const gfc_batch &bt)
 	return a;
 }
 
-// The prime set of every test of the batch, or ANY_SET.
-int common_set(const gfc_batch &bt)
+// The prime sets the kernel of a single-CTA or short cluster launch holds.  A
+// recorded launch stays valid while every test keeps its number of primes, so
+// it holds both two-prime sets wherever the batch uses set 3.  Outside capture
+// a batch all on set 3 takes the kernel of that set alone (one B200, us: one
+// test a call on the cluster plan at n = 12, 13 8.9, 9.4, with both bodies 9.1,
+// 9.6; 64 tests a squaring on the single-CTA plan at n = 12, 13, 14 12.42,
+// 25.7, 44.8, with both 12.48, 25.9, 45.7).
+int launch_sets(const gfc_batch &bt)
 {
-	for (int set : { 0, 1, 3 })
-		if (bt.nset[set] == static_cast<int>(bt.count)) return set;
-	return ANY_SET;
+	if (!bt.capturing && (bt.nset[3] == static_cast<int>(bt.count))) return SETS_3;
+	const int two = bt.nset[0] + bt.nset[3];
+	return ((two > 0) ? (bt.s3 ? SETS_03 : SETS_0) : 0) | ((bt.nset[1] > 0) ? SETS_1 : 0);
 }
 
 // Single-CTA kernel: one launch for all tests.
 void launch_small(const gfc_batch &bt, const Args &a, cudaStream_t s, bool prep)
 {
-	const int grid = static_cast<int>(bt.count);
-	if (prep)      // every variant: an admission may change the sets present
-	{
-		small_set<0>(bt.n, a, grid, s, true);
-		small_set<1>(bt.n, a, grid, s, true);
-		small_set<3>(bt.n, a, grid, s, true);
-		small_set<ANY_SET>(bt.n, a, grid, s, true);
-		return;
-	}
-	switch (common_set(bt))
-	{
-		case 0: small_set<0>(bt.n, a, grid, s, false); break;
-		case 1: small_set<1>(bt.n, a, grid, s, false); break;
-		case 3: small_set<3>(bt.n, a, grid, s, false); break;
-		default: small_set<ANY_SET>(bt.n, a, grid, s, false);
-	}
+	const int grid = static_cast<int>(bt.count), sets = launch_sets(bt);
+	// every variant is prepared: an admission may change the sets present
+	if (prep || (sets == SETS_0)) small_set<SETS_0>(bt.n, a, grid, s, prep);
+	if (prep || (sets == SETS_1)) small_set<SETS_1>(bt.n, a, grid, s, prep);
+	if (prep || (sets == SETS_01)) small_set<SETS_01>(bt.n, a, grid, s, prep);
+	if (prep || (sets == SETS_3)) small_set<SETS_3>(bt.n, a, grid, s, prep);
+	if (prep || (sets == SETS_03)) small_set<SETS_03>(bt.n, a, grid, s, prep);
+	if (prep || (sets == SETS_ANY)) small_set<SETS_ANY>(bt.n, a, grid, s, prep);
 }
 
-// Cluster-resident squarings: one persistent launch over all tests.
+// Cluster-resident squarings: one persistent launch over all tests.  The graphs
+// of the long rows (n >= 15) outlive a change of width, those of the short rows
+// do not: a batch of two-prime tests then takes the kernel of those sets.
 void launch_cluster(gfc_batch &bt, const Args &a, cudaStream_t s)
 {
-	// set 3's own kernel only where a graph is refused once a test has changed set
-	const int set = !bt.s3 ? 0 : (((bt.lr == 0) && (common_set(bt) == 3)) ? 3 : ANY_SET);
-	launch_cluster_n(bt.n, a, static_cast<int>(bt.count), bt.cluster_max, set, s, false, nullptr);
+	const int sets = ((bt.lr == 0) && bt.s3 && (bt.nset[1] == 0)) ? launch_sets(bt) : sets_of(bt.s3);
+	launch_cluster_n(bt.n, a, static_cast<int>(bt.count), bt.cluster_max, sets, s, false, nullptr);
 }
 
 // Raises shared-memory limits of the kernels the current plan uses.
@@ -1207,7 +1209,7 @@ void prepare_plan(gfc_batch &bt)
 		bt.twist = bt.packed ? &get_twist(*bt.tabp, true, bt.lr) : &get_twist(*bt.tab, false, bt.lr);
 	Args a{};
 	a.n = bt.n;
-	if (bt.cluster > 0) launch_cluster_n(bt.n, a, 0, 0, ANY_SET, nullptr, true, &bt.cluster_max);
+	if (bt.cluster > 0) launch_cluster_n(bt.n, a, 0, 0, SETS_ANY, nullptr, true, &bt.cluster_max);
 	if (bt.packed)
 	{
 		launch_pcol(bt.six ? MID_LR1 : bt.lr, true, a, 0, nullptr, true);
@@ -1784,7 +1786,7 @@ void op_admit(gfc_batch &bt, size_t test, uint32_t b, const uint32_t *words, uin
 	materialize(bt);
 	if (s != bt.set[test])
 	{
-		bt.sets_version++;
+		if (set_width(s) != set_width(bt.set[test])) bt.widths_version++;
 		bt.nset[bt.set[test]]--;
 		bt.set[test] = s;
 		bt.nset[s]++;
@@ -2151,7 +2153,7 @@ GFC_API int gfc_batch_assign(gfc_batch *bt, size_t test, uint32_t b)
 		cudaSetDevice(bt->device);
 		materialize(*bt);
 		GFC_CK(cudaStreamSynchronize(bt->stream));
-		if (s != bt->set[test]) bt->sets_version++;
+		if (set_width(s) != set_width(bt->set[test])) bt->widths_version++;
 		bt->nset[bt->set[test]]--;
 		bt->b[test] = b;
 		bt->set[test] = s;
@@ -2358,7 +2360,7 @@ GFC_API int gfc_batch_capture_end(gfc_batch *bt, gfc_graph **out)
 		bt->capturing = false;
 		std::unique_ptr<gfc_graph> g(new gfc_graph());
 		g->batch = bt; g->device = bt->device; g->stream = bt->stream;
-		g->sets_version = bt->sets_version; g->per_set = (bt->lr == 0);
+		g->widths_version = bt->widths_version; g->per_width = (bt->lr == 0);
 		// recorded launches are counted when the graph runs, not here
 		g->kernels = g_launches.load() - bt->capture_start;
 		g_launches.fetch_sub(g->kernels);
@@ -2373,8 +2375,8 @@ GFC_API int gfc_graph_launch(gfc_graph *g)
 	return guard([&] {
 		GFC_NULLCHK(g);
 		cudaSetDevice(g->device);
-		if ((g->batch != nullptr) && g->per_set && (g->batch->sets_version != g->sets_version))
-			fail(GFC_ERR_STATE, "graph_launch: a test changed prime set since capture; capture again");
+		if ((g->batch != nullptr) && g->per_width && (g->batch->widths_version != g->widths_version))
+			fail(GFC_ERR_STATE, "graph_launch: a test changed its number of primes since capture; capture again");
 		if (g->batch != nullptr) materialize(*g->batch);
 		GFC_CK(cudaGraphLaunch(g->exec, g->stream));
 		g_launches.fetch_add(g->kernels);

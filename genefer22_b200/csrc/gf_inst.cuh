@@ -7,23 +7,23 @@
 
 #include "gf_kernels.cuh"
 
-#define GFC_SMALL_N(T, SET, LOGN) T void k_small<SET, LOGN, false>(const Args);
-#define GFC_SMALL_S(T, SET, LOGN) T void k_small<SET, LOGN, true>(const Args);
+#define GFC_SMALL_N(T, SETS, LOGN) T void k_small<SETS, LOGN, false>(const Args);
+#define GFC_SMALL_S(T, SETS, LOGN) T void k_small<SETS, LOGN, true>(const Args);
+#define GFC_SMALL_SETS(G, T, LOGN)                                                                                     \
+	G(T, SETS_0, LOGN) G(T, SETS_1, LOGN) G(T, SETS_01, LOGN) G(T, SETS_3, LOGN) G(T, SETS_03, LOGN) G(T, SETS_ANY, LOGN)
 #define GFC_INST_SMALL(T)                                                                                              \
-	GFC_SMALL_N(T, ANY_SET, 10) GFC_SMALL_S(T, ANY_SET, 10) GFC_SMALL_N(T, ANY_SET, 11) GFC_SMALL_S(T, ANY_SET, 11)    \
-	GFC_SMALL_N(T, 0, 12) GFC_SMALL_S(T, 0, 12) GFC_SMALL_N(T, 1, 12) GFC_SMALL_S(T, 1, 12)                            \
-	GFC_SMALL_N(T, 3, 12) GFC_SMALL_S(T, 3, 12) GFC_SMALL_N(T, ANY_SET, 12) GFC_SMALL_S(T, ANY_SET, 12)                \
-	GFC_SMALL_N(T, 0, 13) GFC_SMALL_N(T, 1, 13) GFC_SMALL_N(T, 3, 13) GFC_SMALL_N(T, ANY_SET, 13)                      \
-	GFC_SMALL_N(T, 0, 14) GFC_SMALL_N(T, 1, 14) GFC_SMALL_N(T, 3, 14) GFC_SMALL_N(T, ANY_SET, 14)
+	GFC_SMALL_N(T, SETS_ANY, 10) GFC_SMALL_S(T, SETS_ANY, 10) GFC_SMALL_N(T, SETS_ANY, 11)                             \
+	GFC_SMALL_S(T, SETS_ANY, 11) GFC_SMALL_SETS(GFC_SMALL_N, T, 12) GFC_SMALL_SETS(GFC_SMALL_S, T, 12)                 \
+	GFC_SMALL_SETS(GFC_SMALL_N, T, 13) GFC_SMALL_SETS(GFC_SMALL_N, T, 14)
 
-#define GFC_CLUSTER(T, LQ, LC, SET) T void k_cluster<LQ, LC, SET>(const Args, int);
-#define GFC_INST_CLUSTER_SHORT(T)                                                                                      \
-	GFC_CLUSTER(T, 3, 9, 0) GFC_CLUSTER(T, 3, 9, 3) GFC_CLUSTER(T, 3, 9, ANY_SET)                                      \
-	GFC_CLUSTER(T, 4, 9, 0) GFC_CLUSTER(T, 4, 9, 3) GFC_CLUSTER(T, 4, 9, ANY_SET)                                      \
-	GFC_CLUSTER(T, 4, 10, 0) GFC_CLUSTER(T, 4, 10, 3) GFC_CLUSTER(T, 4, 10, ANY_SET)
+#define GFC_CLUSTER(T, LQ, LC, SETS) T void k_cluster<LQ, LC, SETS>(const Args, int);
+#define GFC_CLUSTER_S(T, LQ, LC)                                                                                       \
+	GFC_CLUSTER(T, LQ, LC, SETS_01) GFC_CLUSTER(T, LQ, LC, SETS_3) GFC_CLUSTER(T, LQ, LC, SETS_03)                     \
+	GFC_CLUSTER(T, LQ, LC, SETS_ANY)
+#define GFC_INST_CLUSTER_SHORT(T) GFC_CLUSTER_S(T, 3, 9) GFC_CLUSTER_S(T, 4, 9) GFC_CLUSTER_S(T, 4, 10)
 #define GFC_INST_CLUSTER_LONG(T)                                                                                       \
-	GFC_CLUSTER(T, 2, 13, 0) GFC_CLUSTER(T, 2, 13, ANY_SET)                                                            \
-	GFC_CLUSTER(T, 3, 13, 0) GFC_CLUSTER(T, 3, 13, ANY_SET) GFC_CLUSTER(T, 4, 13, 0) GFC_CLUSTER(T, 4, 13, ANY_SET)
+	GFC_CLUSTER(T, 2, 13, SETS_01) GFC_CLUSTER(T, 2, 13, SETS_ANY) GFC_CLUSTER(T, 3, 13, SETS_01)                      \
+	GFC_CLUSTER(T, 3, 13, SETS_ANY) GFC_CLUSTER(T, 4, 13, SETS_01) GFC_CLUSTER(T, 4, 13, SETS_ANY)
 
 #define GFC_COL(T, LR) T void k_col_fwd<LR>(const Args); T void k_col_inv<LR>(const Args);
 #define GFC_INST_COL(T) GFC_COL(T, 5) GFC_COL(T, 6) GFC_COL(T, 7) GFC_COL(T, 8) GFC_COL(T, 9) GFC_COL(T, 10)

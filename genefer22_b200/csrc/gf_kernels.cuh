@@ -100,22 +100,35 @@ __device__ __forceinline__ void for_planes(F &&f)
 
 
 
-// Kernels of unpacked launches come with and without S3: a batch none of whose
-// tests was on set 3 when it was made keeps its tests on sets 0 and 1, and its
-// kernels hold the bodies of those only.  (With the third body in every kernel
-// ptxas takes more registers or another schedule: three-prime batches of 64 at
-// n = 15, 16 measured 1.5-3 % slower on one B200, and equal in this form.)  Set 3 runs set 1's row and middle passes on its
-// first two planes.
-constexpr int ANY_SET = 4;       // template argument of kernels that take each test's set as it comes
+// The prime sets whose bodies an unpacked kernel holds: bit `set` of a mask.
+// A batch none of whose tests was on set 3 when it was made keeps its tests on
+// sets 0 and 1 (SETS_01), and its kernels hold the bodies of those only: with
+// the third body ptxas takes more registers or another schedule (three-prime
+// batches of 64 at n = 15, 16 measured 1.5-3 % slower on one B200, and equal
+// without it).  Set 3 runs set 1's row and middle passes on its first two planes.
+constexpr int SETS_0 = 1, SETS_1 = 2, SETS_01 = 3, SETS_3 = 8, SETS_03 = 9, SETS_ANY = 11;
+__host__ __device__ constexpr int sets_of(bool s3) { return s3 ? SETS_ANY : SETS_01; }
 
 __device__ __forceinline__ int set_planes(int set) { return (set == 1) ? 3 : 2; }
 
-// f(integral_constant<SET>) for the set of a test of an unpacked launch.
-template <bool S3, class F>
+// f(integral_constant<SET>) for the set of a test of an unpacked launch whose
+// tests are on sets of SETS.
+template <int SETS, class F>
 __device__ __forceinline__ void by_set(int set, F &&f)
 {
-	if (set == 0) f(std::integral_constant<int, 0>{});
-	else if (!S3 || (set == 1)) f(std::integral_constant<int, 1>{});
+	constexpr bool S0 = (SETS & 1) != 0, S1 = (SETS & 2) != 0, S3 = (SETS & 8) != 0;
+	if constexpr (S0 && !S1 && !S3) f(std::integral_constant<int, 0>{});
+	else if constexpr (S0)
+	{
+		if (set == 0) f(std::integral_constant<int, 0>{});
+		else by_set<SETS & ~1>(set, f);
+	}
+	else if constexpr (S1 && !S3) f(std::integral_constant<int, 1>{});
+	else if constexpr (S1)
+	{
+		if (set == 1) f(std::integral_constant<int, 1>{});
+		else f(std::integral_constant<int, 3>{});
+	}
 	else f(std::integral_constant<int, 3>{});
 }
 
@@ -686,20 +699,17 @@ __device__ __forceinline__ void small_body(const Args &a, int t, const TestDesc 
 	if ((tid == 0) && (a.op == OP_SQUARE) && (a.dup_mode == DUP_BITS)) a.pos[t] -= done;
 }
 
-// One CTA per test of prime set SET, or with SET = ANY_SET of the set of its
-// test: threads and shared memory are then those of the three-prime set (the
-// threads past a two-prime test's own only join the barriers).  A batch of
-// several sets runs in one launch: with a launch per set the second waited for
-// the first (102 tests at n = 12 of sets 0 and 1, one B200: 31.6 -> 18.5 us per
-// squaring; of one set 15.2 and 16.6, and 2 % more with the code of both in the
-// kernel).
-template <int SET, int LOGN, bool SPLIT>
-struct SmallLaunch : SmallShape<(SET == ANY_SET) ? 1 : SET, LOGN, SPLIT>
+// One CTA per test, of the set of its test; threads and shared memory are those
+// of the widest set of SETS (the threads past a two-prime test's own only join
+// the barriers).  A batch of several sets runs in one launch: with a launch per
+// set the second waited for the first.
+template <int SETS, int LOGN, bool SPLIT>
+struct SmallLaunch : SmallShape<((SETS & SETS_1) != 0) ? 1 : 0, LOGN, SPLIT>
 {
 };
 
-template <int SET, int LOGN, bool SPLIT>
-__global__ void __launch_bounds__(SmallLaunch<SET, LOGN, SPLIT>::T, SmallLaunch<SET, LOGN, SPLIT>::MINB)
+template <int SETS, int LOGN, bool SPLIT>
+__global__ void __launch_bounds__(SmallLaunch<SETS, LOGN, SPLIT>::T, SmallLaunch<SETS, LOGN, SPLIT>::MINB)
 	k_small(const Args a)
 {
 	pdl_wait();
@@ -707,8 +717,7 @@ __global__ void __launch_bounds__(SmallLaunch<SET, LOGN, SPLIT>::T, SmallLaunch<
 	const int t = a.tests[blockIdx.x];
 	if (!test_ok(a, t)) return;
 	const TestDesc &d = a.desc[t];
-	if constexpr (SET != ANY_SET) small_body<SET, LOGN, SPLIT>(a, t, d, sm);
-	else by_set<true>(d.set, [&](auto S) { small_body<decltype(S)::value, LOGN, SPLIT>(a, t, d, sm); });
+	by_set<SETS>(d.set, [&](auto S) { small_body<decltype(S)::value, LOGN, SPLIT>(a, t, d, sm); });
 }
 
 // ------------------------------------------------------------------ k_cluster
@@ -961,9 +970,8 @@ __device__ __forceinline__ void cluster_test(const Args &a, int t, const TestDes
 	if ((tid == 0) && (q == 0) && (a.dup_mode == DUP_BITS)) a.pos[t] = (pos0 - iters < -1) ? -1 : pos0 - iters;
 }
 
-// Persistent grid of clusters over the tests a.tests[0 .. ntests-1]: of sets 0
-// and 1 (SET = 0), all of set 3, or of any (ANY_SET).
-template <int LQ, int LC, int SET>
+// Persistent grid of clusters over the tests a.tests[0 .. ntests-1], of sets of SETS.
+template <int LQ, int LC, int SETS>
 __global__ void __launch_bounds__(ClusterShape<LQ, LC>::T, ClusterShape<LQ, LC>::MINB) k_cluster(const Args a, int ntests)
 {
 	pdl_wait();
@@ -979,12 +987,7 @@ __global__ void __launch_bounds__(ClusterShape<LQ, LC>::T, ClusterShape<LQ, LC>:
 		if (test_ok(a, t))
 		{
 			const TestDesc &d = a.desc[t];
-			if constexpr (SET == 3) cluster_test<3, LQ, LC>(a, t, d, sm, q);
-			else if constexpr (SET == 0)
-			{
-				if (d.set == 0) cluster_test<0, LQ, LC>(a, t, d, sm, q); else cluster_test<1, LQ, LC>(a, t, d, sm, q);
-			}
-			else by_set<true>(d.set, [&](auto S_) { cluster_test<decltype(S_)::value, LQ, LC>(a, t, d, sm, q); });
+			by_set<SETS>(d.set, [&](auto S_) { cluster_test<decltype(S_)::value, LQ, LC>(a, t, d, sm, q); });
 		}
 		// the next test's first shared-memory writes follow this barrier, after
 		// every CTA has read this test's last carries
@@ -1197,7 +1200,7 @@ __global__ void __launch_bounds__(col_threads(LR)) k_col_fwd(const Args a)
 	bool active;
 	(void)get_dup(a, d, t, a.j, active);
 	if (!active) return;
-	by_set<true>(d.set, [&](auto S) { col_fwd_body<decltype(S)::value, LR>(a, d, sm); });
+	by_set<SETS_ANY>(d.set, [&](auto S) { col_fwd_body<decltype(S)::value, LR>(a, d, sm); });
 }
 
 // Rows: the last log2 C forward stages, pointwise, first inverse stages.
@@ -1286,7 +1289,7 @@ __global__ void __launch_bounds__(col_threads(LR)) k_col_inv(const Args a)
 	bool active;
 	const bool dup = get_dup(a, d, t, a.j, active);
 	if (!active) return;
-	by_set<true>(d.set, [&](auto S) { col_inv_body<decltype(S)::value, LR>(a, d, dup, sm); });
+	by_set<SETS_ANY>(d.set, [&](auto S) { col_inv_body<decltype(S)::value, LR>(a, d, dup, sm); });
 }
 
 // ---- transforms of one thread's registers.
@@ -1494,7 +1497,7 @@ __global__ void __launch_bounds__(col_threads(LR2)) k_mid(const Args a)
 	(void)get_dup(a, d, t, a.j, active);
 	if (!active) return;
 	if (d.set == 2) mid_body<2, LR2, INV>(a, d, sm);
-	else by_set<true>(d.set, [&](auto S) { mid_body<decltype(S)::value, LR2, INV>(a, d, sm); });
+	else by_set<SETS_ANY>(d.set, [&](auto S) { mid_body<decltype(S)::value, LR2, INV>(a, d, sm); });
 }
 
 // The middle pass in registers: a thread owns one column of one plane of one
@@ -1772,7 +1775,7 @@ __global__ void __launch_bounds__(COLR_THREADS) k_colr_fwd(const Args a)
 	bool active;
 	(void)get_dup(a, d, t, a.j, active);
 	if (!active) return;
-	by_set<S3>(d.set, [&](auto S) { col_fwd_reg_body<decltype(S)::value, LR>(a, d, sm); });
+	by_set<sets_of(S3)>(d.set, [&](auto S) { col_fwd_reg_body<decltype(S)::value, LR>(a, d, sm); });
 }
 
 template <int LR>
@@ -1791,7 +1794,7 @@ __global__ void __launch_bounds__(COLR_THREADS) k_colr_inv(const Args a)
 	bool active;
 	const bool dup = get_dup(a, d, t, a.j, active);
 	if (!active) return;
-	by_set<S3>(d.set, [&](auto S) { col_inv_reg_body<decltype(S)::value, LR>(a, d, dup, sm); });
+	by_set<sets_of(S3)>(d.set, [&](auto S) { col_inv_reg_body<decltype(S)::value, LR>(a, d, dup, sm); });
 }
 
 // ---- plane-split register columns, for batches too small to fill the GPU
@@ -1894,7 +1897,7 @@ __global__ void __launch_bounds__(WMAX * CS_T) k_colr_fwd_s(const Args a)
 	bool active;
 	(void)get_dup(a, d, t, a.j, active);
 	if (!active) return;
-	by_set<S3>(d.set, [&](auto S) { col_fwd_split_body<decltype(S)::value, LR>(a, d, sm); });
+	by_set<sets_of(S3)>(d.set, [&](auto S) { col_fwd_split_body<decltype(S)::value, LR>(a, d, sm); });
 }
 
 template <int LR, bool S3>
@@ -1907,7 +1910,7 @@ __global__ void __launch_bounds__(WMAX * CS_T) k_colr_inv_s(const Args a)
 	bool active;
 	const bool dup = get_dup(a, d, t, a.j, active);
 	if (!active) return;
-	by_set<S3>(d.set, [&](auto S) { col_inv_split_body<decltype(S)::value, LR>(a, d, dup, sm); });
+	by_set<sets_of(S3)>(d.set, [&](auto S) { col_inv_split_body<decltype(S)::value, LR>(a, d, dup, sm); });
 }
 
 // ---- packed digits (prime set 2).

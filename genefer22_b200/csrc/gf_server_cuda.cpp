@@ -147,7 +147,8 @@ public:
 		int rc = gfc_graph_launch(g_);
 		if (rc == GFC_ERR_STATE)
 		{
-			// a slot changed prime set under the single-CTA plan: record again
+			// a slot changed its number of primes under a plan whose graphs
+			// depend on it: record again
 			gfc_graph_destroy(g_);
 			g_ = nullptr;
 			capture();
@@ -197,8 +198,8 @@ private:
 class CudaCheck : public CheckDev
 {
 public:
-	// The check runs from one CUDA graph (recorded here, again after a change
-	// of prime set under the single-CTA plan): enqueued call by call it is
+	// The check runs from one CUDA graph (recorded here, and again when a
+	// launch of it is refused after a change of width): enqueued call by call it is
 	// thousands of launches at large n, whose queue would hold up the
 	// dispatcher thread until the device drained it.  Every exponent 2^res
 	// is padded to RB bits with leading zeros (squaring 1 keeps 1), so one

@@ -137,9 +137,10 @@ int gfc_batch_set_exponent(gfc_batch *bt, size_t test, const uint32_t *words, ui
 /* Gives slot `test` a new base b (its prime set and carry constants follow);
  * the slot's registers keep their contents until overwritten.  Synchronises.
  * Used to admit a new test into a running batch.  No counterpart in the
- * reference, which runs one test per transform.  With the single-CTA plan
- * (n <= 14) a graph captured before a change of prime set is refused by
- * gfc_graph_launch (GFC_ERR_STATE); four-step graphs stay valid. */
+ * reference, which runs one test per transform.  Under the single-CTA plan and
+ * the cluster plan of n <= 14 a graph captured before a slot changed its number
+ * of primes (2 or 3, gfc_batch_widths) is refused by gfc_graph_launch
+ * (GFC_ERR_STATE); other graphs stay valid. */
 int gfc_batch_assign(gfc_batch *bt, size_t test, uint32_t b);
 
 /* Reserved slots (no counterpart in the reference, which runs one test per
@@ -154,8 +155,8 @@ int gfc_batch_reserve(gfc_batch *bt, uint64_t max_bits);
  * set and carry constants), r_0 = r_1 = 1 (genefer's start, src/genefer.h:492-497),
  * exponent words (nbits <= max_bits) and bit position nbits - 1, as one
  * asynchronous sequence on the batch stream.  `words` may be reused when the
- * call returns.  A change of prime set under the single-CTA plan makes graphs
- * captured before it refuse to launch (GFC_ERR_STATE), as gfc_batch_assign. */
+ * call returns.  A change of the slot's number of primes makes graphs of the
+ * plans gfc_batch_assign names refuse to launch (GFC_ERR_STATE). */
 int gfc_batch_admit(gfc_batch *bt, size_t test, uint32_t b, const uint32_t *words, uint64_t nbits);
 
 /* Register `reg` of one test to / from host memory, enqueued on the batch

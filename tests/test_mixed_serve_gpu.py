@@ -51,13 +51,13 @@ def test_assign_changes_base_and_set(oracle):
 
 
 def test_graph_refused_after_set_change():
-    """Single-CTA graphs launch per prime set: a change of set since capture
-    is refused; four-step graphs stay valid."""
+    """Single-CTA graphs hold the kernels of the widths present: a change of a
+    test's number of primes since capture is refused; four-step graphs stay valid."""
     bt = Batch([1_000_002, 1_999_999_998], 12)
     g = bt.capture(lambda: bt.square(False, 2))
     bt.assign(0, 1_000_004)               # same set: still valid
     g.launch()
-    bt.assign(0, 1_999_999_990)           # set 0 -> set 1
+    bt.assign(0, 1_999_999_990)           # two primes -> three
     with pytest.raises(GfcError):
         g.launch()
     g.close()

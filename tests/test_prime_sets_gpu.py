@@ -4,7 +4,7 @@ against the oracle, on every shape of plan."""
 import numpy as np
 import pytest
 
-from genefer22_b200 import Batch, Transform, gint
+from genefer22_b200 import Batch, GfcError, Transform, gint
 
 pytestmark = pytest.mark.gpu
 
@@ -57,4 +57,76 @@ def test_mixed_sets(oracle, n, plan):
         for _ in range(3):
             o.squareDup(True)
         assert np.array_equal(gint.unbalance(bt.get(i), b), gint.unbalance(o.getInt(), b)), i
+    bt.close()
+
+
+def _load(oracle, bt, seed):
+    """Seeded digits in register 0 of every test, and oracles that hold the same."""
+    rng = np.random.default_rng(seed)
+    oracles = []
+    for i, b in enumerate(int(x) for x in bt.bases):
+        d = rng.integers(-(b // 2), b // 2 + 1, 1 << bt.n).astype(np.int32)
+        bt.put(i, d)
+        oracles.append(oracle.OracleTransform(b, bt.n))
+        oracles[-1].setInt(d)
+    return oracles
+
+
+def _squared(bt, oracles, run, times):
+    """run() squares register 0 of every test `times` times with dup."""
+    run()
+    for i, (o, b) in enumerate(zip(oracles, bt.bases)):
+        for _ in range(times):
+            o.squareDup(True)
+        assert np.array_equal(gint.unbalance(bt.get(i), int(b)), gint.unbalance(o.getInt(), int(b))), i
+
+
+@pytest.mark.parametrize("n,plan", [(10, 0), (11, 0), (12, 0), (12, 1), (13, 0), (13, 1), (14, 0), (14, 1)])
+def test_graph_outlives_a_move_between_the_two_prime_sets(oracle, n, plan):
+    """A graph recorded with every test on one two-prime set serves a test that
+    moves to the other one; a change of width is refused until a new capture."""
+    low, high, wide = 1026, top_base(n) + 2, 1_999_999_998
+    bt = Batch([low, low + 2], n)
+    bt.set_plan(plan)
+    g = bt.capture(lambda: bt.square(True, 2))
+    for slot, b in ((0, high), (1, high + 2), (0, low)):
+        bt.assign(slot, b)
+        assert list(bt.widths()) == [2, 2]
+        _squared(bt, _load(oracle, bt, b % 97), g.launch, 2)
+        _squared(bt, _load(oracle, bt, b % 89), lambda: bt.square(True, 2), 2)
+    bt.assign(1, wide)
+    with pytest.raises(GfcError):
+        g.launch()
+    g.close()
+    g = bt.capture(lambda: bt.square(True, 2))
+    _squared(bt, _load(oracle, bt, 5), g.launch, 2)
+    _squared(bt, _load(oracle, bt, 6), lambda: bt.square(True, 2), 2)
+    g.close()
+    bt.close()
+
+
+@pytest.mark.parametrize("n,plan", [(12, 0), (12, 1), (13, 3), (14, 5), (15, 1), (16, 4), (18, 103)])
+@pytest.mark.parametrize("width", [2, 3])
+def test_small_base_in_a_batch_made_without_one(oracle, n, plan, width):
+    """A batch made without a base of set 3's range has kernels without its body:
+    a small base that comes later (assign, admit) stays on the 32-bit primes."""
+    b0 = top_base(n) + 2 if width == 2 else 1_999_999_998 if n <= 15 else 999_999_998
+    bt = Batch([b0, b0 + 2], n)
+    bt.set_plan(plan)
+    assert list(bt.widths()) == [width] * 2
+    g = bt.capture(lambda: bt.square(True, 2)) if plan > 1 or width == 2 else None
+    bt.assign(0, 1026)
+    _squared(bt, _load(oracle, bt, n), lambda: bt.square(True, 2), 2)
+    if g is not None:
+        _squared(bt, _load(oracle, bt, n + 1), g.launch, 2)
+        g.close()
+    bt.reserve(64)
+    bt.admit(1, 2050, np.array([0b1011], np.uint32), 4)
+    bt.assign(0, b0)
+    bt.square_exp(4)
+    o = oracle.OracleTransform(2050, n)
+    o.set(1)
+    for bit in (True, False, True, True):
+        o.squareDup(bit)
+    assert np.array_equal(gint.unbalance(bt.get(1), 2050), gint.unbalance(o.getInt(), 2050))
     bt.close()
