@@ -560,18 +560,16 @@ int sm_count()
 template <int SETS, int LOGN>
 void small_t(const Args &a, int grid, cudaStream_t s, bool prep)
 {
-	// n = 10, 11 have the kernel of any set only
-	constexpr int ST = (LOGN >= 12) ? SETS : SETS_ANY;
-	using L = SmallLaunch<ST, LOGN, false>;
-	using LS = SmallLaunch<ST, LOGN, true>;
-	if (prep) set_smem(k_small<ST, LOGN, false>, L::SMEM);
+	using L = SmallLaunch<SETS, LOGN, false>;
+	using LS = SmallLaunch<SETS, LOGN, true>;
+	if (prep) set_smem(k_small<SETS, LOGN, false>, L::SMEM);
 	if constexpr (LS::PSPLIT)
 	{
 		// fewer tests than SMs: plane-split passes (more warps per test)
-		if (prep) set_smem(k_small<ST, LOGN, true>, LS::SMEM);
-		else if (grid < sm_count()) { launch_pdl(k_small<ST, LOGN, true>, dim3(grid), dim3(LS::T), LS::SMEM, s, a); return; }
+		if (prep) set_smem(k_small<SETS, LOGN, true>, LS::SMEM);
+		else if (grid < sm_count()) { launch_pdl(k_small<SETS, LOGN, true>, dim3(grid), dim3(LS::T), LS::SMEM, s, a); return; }
 	}
-	if (!prep) launch_pdl(k_small<ST, LOGN, false>, dim3(grid), dim3(L::T), L::SMEM, s, a);
+	if (!prep) launch_pdl(k_small<SETS, LOGN, false>, dim3(grid), dim3(L::T), L::SMEM, s, a);
 }
 
 template <int SETS>

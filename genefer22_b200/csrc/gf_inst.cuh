@@ -12,8 +12,8 @@
 #define GFC_SMALL_SETS(G, T, LOGN)                                                                                     \
 	G(T, SETS_0, LOGN) G(T, SETS_1, LOGN) G(T, SETS_01, LOGN) G(T, SETS_3, LOGN) G(T, SETS_03, LOGN) G(T, SETS_ANY, LOGN)
 #define GFC_INST_SMALL(T)                                                                                              \
-	GFC_SMALL_N(T, SETS_ANY, 10) GFC_SMALL_S(T, SETS_ANY, 10) GFC_SMALL_N(T, SETS_ANY, 11)                             \
-	GFC_SMALL_S(T, SETS_ANY, 11) GFC_SMALL_SETS(GFC_SMALL_N, T, 12) GFC_SMALL_SETS(GFC_SMALL_S, T, 12)                 \
+	GFC_SMALL_SETS(GFC_SMALL_N, T, 10) GFC_SMALL_SETS(GFC_SMALL_S, T, 10) GFC_SMALL_SETS(GFC_SMALL_N, T, 11)           \
+	GFC_SMALL_SETS(GFC_SMALL_S, T, 11) GFC_SMALL_SETS(GFC_SMALL_N, T, 12) GFC_SMALL_SETS(GFC_SMALL_S, T, 12)           \
 	GFC_SMALL_SETS(GFC_SMALL_N, T, 13) GFC_SMALL_SETS(GFC_SMALL_N, T, 14)
 
 #define GFC_CLUSTER(T, LQ, LC, SETS) T void k_cluster<LQ, LC, SETS>(const Args, int);

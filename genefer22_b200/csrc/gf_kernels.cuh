@@ -612,7 +612,8 @@ struct SmallShape
 	static constexpr size_t SMEM = size_t(W) * PN * 4 + size_t(T) * 8;
 };
 
-template <int SET, int LOGN, bool SPLIT>
+// T: threads of the launch (the kernel's widest set's).
+template <int SET, int LOGN, bool SPLIT, int T>
 __device__ __forceinline__ void small_body(const Args &a, int t, const TestDesc &d, uint32_t *sm)
 {
 	using S = SmallShape<SET, LOGN, SPLIT>;
@@ -662,7 +663,7 @@ __device__ __forceinline__ void small_body(const Args &a, int t, const TestDesc 
 		{
 #pragma unroll
 			for (int pl = 0; pl < PrimeSet<SET>::W; ++pl)
-				for (int i = tid; i < N; i += static_cast<int>(blockDim.x)) d.zp[pl * N + i] = sm[pl * PN + MP::addr(i, 0)];
+				for (int i = tid; i < N; i += T) d.zp[pl * N + i] = sm[pl * PN + MP::addr(i, 0)];
 			return;
 		}
 
@@ -717,7 +718,9 @@ __global__ void __launch_bounds__(SmallLaunch<SETS, LOGN, SPLIT>::T, SmallLaunch
 	const int t = a.tests[blockIdx.x];
 	if (!test_ok(a, t)) return;
 	const TestDesc &d = a.desc[t];
-	by_set<SETS>(d.set, [&](auto S) { small_body<decltype(S)::value, LOGN, SPLIT>(a, t, d, sm); });
+	by_set<SETS>(d.set, [&](auto S) {
+		small_body<decltype(S)::value, LOGN, SPLIT, SmallLaunch<SETS, LOGN, SPLIT>::T>(a, t, d, sm);
+	});
 }
 
 // ------------------------------------------------------------------ k_cluster

@@ -1,5 +1,7 @@
-"""Batches at n = 10..14: both prime sets in one single-CTA launch, and the
-default plans by number of tests."""
+"""Batches at n = 10..14: every mix of prime sets in one single-CTA launch, and
+the default plans by number of tests."""
+import math
+
 import numpy as np
 import pytest
 
@@ -27,16 +29,50 @@ def _squared(bases, n, plan, steps=3):
     return out
 
 
-# 150 tests: more than SMs, the CTAs without plane-split passes
-@pytest.mark.parametrize("n,count", [(10, 3), (11, 4), (12, 3), (12, 150), (13, 2), (14, 2)])
-def test_both_sets_in_one_launch(n, count):
-    bases = [(B3, B2)[i % 2] for i in range(count)]
-    got, ref = _squared(bases, n, 0), _squared(bases, n, 3 if n > 10 else 0)
-    for i, b in enumerate(bases):
-        assert np.array_equal(got[i], ref[i]), i
-    one = {b: _squared([b], n, 0)[0] for b in (B2, B3)} if n == 10 else {}
-    if one:                                 # n = 10 has no other plan: a lone test is its own reference
-        assert np.array_equal(got[0], one[B3])
+def _base(n, prime_set):
+    """A base of prime set 3 (two 31-bit primes), 0 (two 32-bit primes) or 1 (three primes) at size n."""
+    m3 = (127 * 2**24 + 1) * (63 * 2**25 + 1)
+    return {3: 1_026, 0: 2 * math.isqrt((m3 // 2) >> n), 1: B3}[prime_set]
+
+
+# 160 tests: more than SMs, the CTAs without plane-split passes
+@pytest.mark.parametrize("sets", [(3,), (0,), (1,), (3, 0), (0, 1), (3, 1), (3, 0, 1)])
+@pytest.mark.parametrize("n,count", [(10, 4), (10, 160), (11, 4), (11, 160), (12, 4), (12, 160), (13, 4), (14, 4)])
+@pytest.mark.parametrize("made", ["at once", "by assign"])
+def test_both_sets_in_one_launch(oracle, n, count, sets, made):
+    """One single-CTA launch over tests of any prime sets; tests moved from set 3
+    leave a batch whose kernels hold its body beside theirs."""
+    bases = [_base(n, sets[i % len(sets)]) for i in range(count)]
+    if made == "at once":
+        bt = Batch(bases, n)
+    else:
+        bt = Batch([_base(n, 3)] * count, n)
+        for i, b in enumerate(bases):
+            bt.assign(i, b)
+    bt.set_plan(0)
+    rng = np.random.default_rng(n)
+    digits = {b: rng.integers(-(b // 2), b // 2 + 1, 1 << n).astype(np.int32) for b in bases}
+    bt.put_all(np.stack([digits[b] for b in bases]))
+    bt.copy(1, 0)
+    bt.square(True, 2)
+    g = bt.capture(lambda: bt.square(False, 2))
+    g.launch()
+    bt.init_multiplicand(1)
+    bt.mul_into(0)
+    got = bt.get_all(0)
+    g.close()
+    bt.close()
+    for b, d in digits.items():
+        o = oracle.OracleTransform(b, n)
+        o.setInt(d)
+        o.copy(1, 0)
+        for dup in (True, True, False, False):
+            o.squareDup(dup)
+        o.initMultiplicand(1)
+        o.mul()
+        ref = gint.unbalance(o.getInt(), b)
+        for i in range(count):
+            assert bases[i] != b or np.array_equal(gint.unbalance(got[i], b), ref), i
 
 
 @pytest.mark.parametrize("n,bases,plan", [
