@@ -703,7 +703,9 @@ __device__ __forceinline__ void small_body(const Args &a, int t, const TestDesc 
 // One CTA per test, of the set of its test; threads and shared memory are those
 // of the widest set of SETS (the threads past a two-prime test's own only join
 // the barriers).  A batch of several sets runs in one launch: with a launch per
-// set the second waited for the first.
+// set the second waited for the first (one B200, graph replay, 102 tests of any
+// base at n = 12 32.3 -> 17.9 us per squaring, with the tests listed by set; of
+// one set 12.4 (3), 15.4 (0) and 17.0 (1)).
 template <int SETS, int LOGN, bool SPLIT>
 struct SmallLaunch : SmallShape<((SETS & SETS_1) != 0) ? 1 : 0, LOGN, SPLIT>
 {
