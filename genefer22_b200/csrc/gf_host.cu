@@ -919,20 +919,52 @@ int default_plan(int n)
 	return PLAN_SIX + lr2[n];
 }
 
+// Clusters of plan 1 at size n that the device holds at once, of whichever of
+// its kernels holds fewest (48, 14 and 7 at n = 12, 13, 14 on a B200: how many
+// fit depends on the SMs of each GPC).
+size_t clusters_at_once(int n)
+{
+	static std::atomic<int> cache[64][24] = {};
+	int dev = 0;
+	GFC_CK(cudaGetDevice(&dev));
+	std::atomic<int> &c = cache[dev & 63][n];
+	int v = c.load();
+	if (v == 0)
+	{
+		Args a{};
+		a.n = n;
+		launch_cluster_n(n, a, 0, 0, SETS_ANY, nullptr, true, &v);
+		c.store(v);
+	}
+	return static_cast<size_t>(v);
+}
+
 // Default plan of `count` tests at n = 12..14 (nset: tests per prime set), from
-// the time of one batch squaring under every plan (graph replay on one B200, us).
-// The cluster plan (8 or 16 CTAs a test) until its CTAs crowd the SMs or the
-// 16-CTA clusters a second wave: n = 12, single-CTA -> cluster, 48 tests 15.0 ->
-// 9.8, 52 tests 15.1 -> 15.5; n = 13, four-step -> cluster, 12 tests 15.1 -> 9.2,
-// 16 tests 16.2 -> 17.4; n = 14 7 tests 15.8 -> 10.3, 8 tests 16.1 -> 20.4.  Then one
-// CTA per test at n = 12 (102 tests: 15.2, four-step 26.3); at n = 13, 14 one CTA's
-// transform is long, and the four-step plan (lr = 3) spreads it: n = 13 51 tests
-// 31.2 -> 22.4, n = 14 38 tests 62.8 -> 29.0.  Wide batches of one prime set keep one
-// CTA per test (n = 13 128 tests 31.3, four-step 35.9; n = 14 62.6, 61.0).
+// the time of one batch squaring under every plan (graph replay on one B200, us,
+// for tests on set 3 / set 0 / three primes / any base):
+//  - the cluster plan while all its clusters run at once, up to 48, 12 and 7
+//    tests: 48 at n = 12 8.8 / 10.0 / 11.0 / 9.9 (single-CTA 12.6 / 15.5 / 17.1 / 18.0),
+//    49 14.4 / 15.2 / 16.4 / 15.4; 12 at n = 13 8.4 / 9.3 / 9.5 / 9.2 (four-step 16.4 /
+//    16.2 / 17.6 / 17.1), 15 15.3 / 17.5 / 17.4 / 17.0; 7 at n = 14 8.9 / 10.3 / 10.2 /
+//    10.2 (17.4 / 17.2 / 18.1 / 18.4), 8 17.4 / 20.4 / 20.2 / 19.0;
+//  - then one CTA per test at n = 12 (102 tests 12.6 / 15.5 / 17.1 / 18.1, four-step
+//    22.0 / 27.9 / 26.1 / 24.3); at n = 13, 14 one CTA's transform is long, and the
+//    four-step plan (lr = 3) spreads it: 63 tests at n = 13 21.9 / 26.8 / 25.0 / 24.1
+//    (single-CTA 26.1 / 31.2 / 33.9 / 34.4), at n = 14 31.4 / 41.4 / 38.2 / 34.1
+//    (45.0 / 62.8 / 62.1 / 64.6); of both widths also beyond: 128 tests 33.4 (34.6)
+//    and 53.4 (64.6);
+//  - 64 tests of one width and more keep the single-CTA plan, and 13 and 14 tests
+//    at n = 13 the four-step one.  Those two lines are choices and no measurements:
+//    the counts had these defaults before, and programs may count on them.
+//    Four-step is faster up to about 96 tests at n = 13 (24.9 / 31.0 / 30.1,
+//    single-CTA 26.1 / 31.2 / 33.9) and 128 at n = 14 (64.5 / 62.4 on set 0 and three
+//    primes, 63.0 / 62.3; set 3 96 tests 41.1, 45.0), the cluster for the others
+//    (14 tests 8.4 / 9.3 / 9.4 / 9.2, four-step 16.6 / 17.1 / 17.8 / 18.5):
+//    gfc_batch_tune takes them.
 int default_small_plan(int n, size_t count, const int (&nset)[4])
 {
-	static const size_t cluster_max[3] = { 48, 12, 7 };
-	if (count <= cluster_max[n - 12]) return PLAN_CLUSTER;
+	static const size_t cluster_tests[3] = { 48, 12, 7 };
+	if ((count <= cluster_tests[n - 12]) && (count <= clusters_at_once(n))) return PLAN_CLUSTER;
 	if ((n >= 13) && ((count < 64) || ((nset[1] > 0) && (nset[1] < static_cast<int>(count))))) return 3;
 	return 0;
 }

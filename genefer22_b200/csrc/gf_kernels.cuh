@@ -762,7 +762,10 @@ struct ClusterShape
 	static constexpr int D = PS ? SEG / 2 : SEG;
 	static constexpr int T0 = C / D;                      // owner threads
 	static constexpr int T = PS ? WMAX * C / 8 : T0;
-	static constexpr int MINB = PS ? 1 : 2;
+	// three CTAs per SM at n = 12: 96 registers, 48 clusters at once (the kernel
+	// of any set took 105, which left 33: 34 to 48 tests a second wave, 8.9 ->
+	// 14 us per squaring of a batch of any set on one B200)
+	static constexpr int MINB = !PS ? 2 : ((LQ == 3) ? 3 : 1);
 	// planes, the owners' carries, and (PS) a fourth word per digit for the
 	// two-stage CRT
 	static constexpr size_t SMEM = size_t(WMAX) * PC * 4 + size_t(T0) * 8 + (PS ? size_t(PC) * 4 : 0);

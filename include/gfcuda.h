@@ -224,9 +224,12 @@ int gfc_batch_set_all(gfc_batch *bt, size_t reg, const int32_t *in);
  * four-step at n = 15, 16 (lr = n - 12), six-step above (103 at n = 17, 18,
  * 104 at n = 19, 20, 105 at n = 21, 106 at n = 22, 107 at n = 23; a lone test at
  * n = 19 too, packed or not); at n = 12..14 up to 48, 12 and 7 tests the cluster
- * plan, and at n = 13, 14 four-step (lr = 3) for fewer than 64 tests and for
- * batches of both widths: the fastest plans measured on one B200.
- * gfc_batch_plan reads the current plan. */
+ * plan (fewer where the device does not hold as many clusters at once), and at
+ * n = 13, 14 four-step (lr = 3) for fewer than 64 tests and for batches of both
+ * widths.  Most are the fastest plans measured on one B200; from 64 tests of one
+ * width at n = 13, 14 the default stays single-CTA where four-step is faster up
+ * to about 96 and 128 tests, and packed digits are no default below n = 16:
+ * gfc_batch_tune sets the fastest.  gfc_batch_plan reads the current plan. */
 int gfc_batch_set_plan(gfc_batch *bt, int lr);
 int gfc_batch_plan(const gfc_batch *bt);
 

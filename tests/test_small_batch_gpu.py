@@ -1,6 +1,7 @@
 """Batches at n = 10..14: every mix of prime sets in one single-CTA launch, and
 the default plans by number of tests."""
 import math
+import time
 
 import numpy as np
 import pytest
@@ -85,3 +86,52 @@ def test_default_small_plans(n, bases, plan):
     if len(bases) <= 13:
         got, ref = _squared(bases, n, None), _squared(bases, n, 0)
         assert all(np.array_equal(g, r) for g, r in zip(got, ref))
+
+
+@pytest.mark.parametrize("n", [12, 13, 14])
+def test_cluster_default_while_every_cluster_runs_at_once(oracle, n):
+    """The last number of tests on the cluster plan and the first one past it square
+    right, of every prime set, and the last takes no second wave of clusters."""
+    plans = {}
+    for count in range(1, 64):
+        bt = Batch([B2] * count, n, num_regs=1)
+        plans[count] = bt.plan()
+        bt.close()
+    last = max(c for c, p in plans.items() if p == 1)
+    assert all(plans[c] == 1 for c in range(1, last + 1))
+    d = {}
+    for count in (last, last + 1):
+        bases = [_base(n, (3, 0, 1)[i % 3]) for i in range(count)]
+        bt = Batch(bases, n)
+        rng = np.random.default_rng(n)
+        for i, b in enumerate(bases):
+            d.setdefault(b, rng.integers(-(b // 2), b // 2 + 1, 1 << n).astype(np.int32))
+            bt.put(i, d[b])
+        bt.square(True, 2)
+        got = bt.get_all(0)
+        bt.close()
+        for b in d:
+            o = oracle.OracleTransform(b, n)
+            o.setInt(d[b])
+            o.squareDup(True)
+            o.squareDup(True)
+            ref = gint.unbalance(o.getInt(), b)
+            assert all(bases[i] != b or np.array_equal(gint.unbalance(got[i], b), ref) for i in range(count))
+
+    def us(count):
+        bt = Batch([B2] * count, n)
+        bt.set_plan(1)
+        g = bt.capture(lambda: bt.square(False, 400))
+        best = 1e9
+        for _ in range(5):
+            bt.sync()
+            t0 = time.perf_counter()
+            g.launch()
+            bt.sync()
+            best = min(best, time.perf_counter() - t0)
+        g.close()
+        bt.close()
+        return best
+
+    one, full = us(1), us(last)
+    assert full < 1.8 * one, (one, full)      # a second wave takes twice the time
