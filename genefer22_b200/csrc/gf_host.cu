@@ -1006,7 +1006,7 @@ struct gfc_batch
 	size_t N = 0, count = 0, num_regs = 0;
 	std::vector<uint32_t> b;
 	std::vector<int> set;
-	bool s3 = false;              // a base of the batch was in set 3's range when it was made: its tests may use it
+	bool s3 = false;              // tests in set 3's range use it (set3_pays when the batch was made)
 	int lr = 0;
 	std::shared_ptr<DeviceTables> tab;
 	void *mem = nullptr;
@@ -1550,6 +1550,32 @@ void check_digits(const gfc_batch &bt, size_t test, const int32_t *in)
 	if (bad != 0) fail(GFC_ERR_ARG, "digits must satisfy |d| <= b/2 + 1 (balance them first)");
 }
 
+// Whether the tests of a new batch that set 3 can hold (nset[3]) use it; set 0
+// holds them too.  A batch all in its range does.  Beside others a test on set
+// 3 ends no earlier than the slowest of its launch, and the launch fetches one
+// more body, so that it pays where work bounds a launch and not latency (one
+// B200, us per squaring in a graph, tests listed by set, without -> with):
+//  - tests of both two-prime sets: the single-CTA plan from the second wave of
+//    CTAs (n = 12 102 tests 15.5 -> 16.4, 160 27.5 -> 23.4), four- and six-step
+//    plans from 2^18 digits (n = 13 20 tests 18.2 -> 19.7, 40 21.8 -> 20.4; n = 14 12
+//    tests 18.2 -> 20.4, 20 24.4 -> 22.8; n = 15 4 tests 18.2 -> 18.9, 8 24.4 -> 22.9;
+//    n = 16 4 tests 25.5 -> 23.7);
+//  - two- and three-prime tests: every plan (n = 12 102 tests 18.5 -> 17.9, n = 13
+//    20 20.5 -> 18.7, n = 15 16 29.8 -> 26.8; 8 at n = 15 and 4 at n = 16 lose 3 and 6 %
+//    in a graph and gain as much in single calls) but the cluster plan at n = 13,
+//    14 (n = 14 4 tests, one call each, 13.3 -> 14.6);
+//  - n = 10, 11: neither (n = 11 64 tests of the two-prime sets 9.1 -> 10.5; 64 of
+//    any base, one call each, 13.8 -> 14.2; 160 at n = 10 12.7 -> 15.7).
+bool set3_pays(const gfc_batch &bt)
+{
+	if ((bt.nset[3] == 0) || (bt.nset[3] == static_cast<int>(bt.count))) return bt.nset[3] > 0;
+	if (bt.n < 12) return false;
+	const int plan = (bt.n <= SMALL_MAX_LOGN) ? default_small_plan(bt.n, bt.count, bt.nset) : default_plan(bt.n);
+	if (plan == PLAN_CLUSTER) return (bt.n == 12) && (bt.nset[1] > 0);
+	if (bt.nset[1] > 0) return true;
+	return (plan == 0) ? (bt.count > static_cast<size_t>(sm_count())) : ((bt.count << bt.n) >= (size_t(1) << 18));
+}
+
 // The launches' list of tests in the order of prime sets 0, 3, 1: tests of one
 // set run side by side.  Neighbouring SMs then fetch the same body, and the
 // wider tests, which come last, fill the launch's tail: against the order the
@@ -1583,11 +1609,17 @@ gfc_batch *batch_create(const uint32_t *b, size_t count, uint32_t n, size_t num_
 		if (s < 0) fail(GFC_ERR_RANGE, "(b, n) is outside the exact range of the RNS prime sets");
 		bt->set[i] = s;
 		bt->nset[s]++;
-		bt->s3 |= (s == 3);
 	}
 	apply_plan(*bt, default_plan(bt->n));
 
 	GFC_CK(cudaSetDevice(device));
+	bt->s3 = set3_pays(*bt);
+	if (!bt->s3)
+	{
+		for (int &s : bt->set) if (s == 3) s = 0;
+		bt->nset[0] += bt->nset[3];
+		bt->nset[3] = 0;
+	}
 	if (stream != nullptr) bt->stream = static_cast<cudaStream_t>(stream);
 	else { GFC_CK(cudaStreamCreateWithFlags(&bt->stream, cudaStreamNonBlocking)); bt->own_stream = true; }
 	bt->tab = get_tables(device, bt->n);

@@ -101,11 +101,14 @@ __device__ __forceinline__ void for_planes(F &&f)
 
 
 // The prime sets whose bodies an unpacked kernel holds: bit `set` of a mask.
-// A batch none of whose tests was on set 3 when it was made keeps its tests on
-// sets 0 and 1 (SETS_01), and its kernels hold the bodies of those only: with
-// the third body ptxas takes more registers or another schedule (three-prime
-// batches of 64 at n = 15, 16 measured 1.5-3 % slower on one B200, and equal
-// without it).  Set 3 runs set 1's row and middle passes on its first two planes.
+// A batch made without tests on set 3 (set3_pays) keeps its tests on sets 0 and
+// 1, and its kernels hold the bodies of those only (SETS_01): with the third
+// body ptxas takes more registers or another schedule (three-prime batches of
+// 64 at n = 15, 16 measured 1.5-3 % slower on one B200, and equal without it).
+// The shared-memory columns (k_col_*) and the 2^7-row middle pass (k_mid<7>)
+// exist with every body alone: one three-prime test at n = 23 (plan 107) takes
+// 410 us per squaring with and 409 without it.  Set 3 runs set 1's row and middle
+// passes on its first two planes.
 constexpr int SETS_0 = 1, SETS_1 = 2, SETS_01 = 3, SETS_3 = 8, SETS_03 = 9, SETS_ANY = 11;
 __host__ __device__ constexpr int sets_of(bool s3) { return s3 ? SETS_ANY : SETS_01; }
 
