@@ -115,6 +115,7 @@ SIGNATURES = {
     "gfc_batch_set_plan": (ctypes.c_int, [vp, ctypes.c_int]),
     "gfc_batch_plan": (ctypes.c_int, [vp]),
     "gfc_batch_widths": (ctypes.c_int, [vp, c_i32p]),
+    "gfc_batch_prime_sets": (ctypes.c_int, [vp, c_i32p]),
     "gfc_batch_sync": (ctypes.c_int, [vp]),
     "gfc_batch_time_kernels": (ctypes.c_int, [vp, ctypes.c_uint32, ctypes.POINTER(ctypes.c_float)]),
     "gfc_batch_stream": (vp, [vp]),

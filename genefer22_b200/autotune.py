@@ -25,8 +25,8 @@ captures K squarings of each candidate plan into a CUDA graph, replays it
 between CUDA events and keeps the fastest (device time per squaring, the
 minimum over a few replays).  It squares register 0 of the batch in place, so
 tune a batch before loading its tests.  This module caches the choice per
-(n, test count, tests on the 3-prime set, packed range) in memory and,
-optionally, in a JSON file.
+(n, test count, tests on each prime set, packed range) in memory and,
+optionally, in a JSON file, whose entries of other kernels are measured again.
 """
 from __future__ import annotations
 
@@ -48,6 +48,10 @@ PLAN_CLUSTER = 1
 PLAN_SIX = 100
 PLAN_PACKED = 200
 PLAN_PACKED_SIX = 300
+
+# Raised when the engine's kernels change so that plans measured before are no
+# guide: entries of a cache file without it are not used (1: no prime set 3).
+KERNELS = 2
 
 
 def packed_ok(b: int, n: int) -> bool:
@@ -74,13 +78,14 @@ class TuneResult:
     us: Dict[int, float] = field(default_factory=dict)   # plan -> microseconds per batch squaring
 
     packable: bool = False
+    low: int = 0                    # tests on two primes below 2^32 (the others' two are below 2^31)
 
     def key(self) -> str:
-        return key(self.n, self.count, self.wide, self.packable)
+        return key(self.n, self.count, self.wide, self.packable, self.low)
 
 
-def key(n: int, count: int, wide: int, packable: bool = False) -> str:
-    return f"n{n}_c{count}_w{wide}" + ("_p" if packable else "")
+def key(n: int, count: int, wide: int, packable: bool = False, low: int = 0) -> str:
+    return f"n{n}_c{count}_w{wide}" + (f"_l{low}" if low else "") + ("_p" if packable else "")
 
 
 class Autotuner:
@@ -91,7 +96,7 @@ class Autotuner:
         self.cache: Dict[str, dict] = {}
         if cache_path and os.path.exists(cache_path):
             with open(cache_path) as f:
-                self.cache = json.load(f)
+                self.cache = {k: c for k, c in json.load(f).items() if c.get("kernels") == KERNELS}
 
     def _save(self):
         if self.cache_path:
@@ -103,14 +108,15 @@ class Autotuner:
     def tune(self, bt: Batch, force: bool = False) -> TuneResult:
         """Chooses and sets the fastest plan for bt (before its tests are loaded)."""
         packable = all(packed_ok(b, bt.n) for b in bt.bases)
-        wide = int(np.count_nonzero(bt.widths() >= 3))
-        k = key(bt.n, bt.count, wide, packable)
+        sets = bt.prime_sets()
+        wide, low = int(np.count_nonzero(sets == 1)), int(np.count_nonzero(sets == 0))
+        k = key(bt.n, bt.count, wide, packable, low)
         if (not force) and (k in self.cache):
             c = self.cache[k]
             try:
                 bt.set_plan(int(c["lr"]))
                 return TuneResult(bt.n, bt.count, wide, int(c["lr"]), {int(a): v for a, v in c["us"].items()},
-                                  packable)
+                                  packable, low)
             except GfcError:
                 pass                                  # a plan this batch cannot take: measure
         plans = (ctypes.c_int32 * 32)()
@@ -121,6 +127,6 @@ class Autotuner:
                                    ctypes.byref(bestc)))
         us: Dict[int, float] = {int(plans[i]): float(times[i]) for i in range(min(cnt.value, 32))}
         best = int(bestc.value)
-        self.cache[k] = {"lr": best, "us": {str(a): v for a, v in us.items()}}
+        self.cache[k] = {"lr": best, "us": {str(a): v for a, v in us.items()}, "kernels": KERNELS}
         self._save()
-        return TuneResult(bt.n, bt.count, wide, best, us, packable)
+        return TuneResult(bt.n, bt.count, wide, best, us, packable, low)

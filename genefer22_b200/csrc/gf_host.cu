@@ -2404,6 +2404,14 @@ GFC_API int gfc_batch_widths(const gfc_batch *bt, int32_t *w)
 	});
 }
 
+GFC_API int gfc_batch_prime_sets(const gfc_batch *bt, int32_t *s)
+{
+	return guard([&] {
+		GFC_NULLCHK(bt); GFC_NULLCHK(s);
+		for (size_t i = 0; i < bt->count; ++i) s[i] = bt->set[i];
+	});
+}
+
 GFC_API int gfc_batch_time_kernels(gfc_batch *bt, uint32_t reps, float *ms)
 {
 	return guard([&] { GFC_NULLCHK(bt); GFC_NULLCHK(ms); cudaSetDevice(bt->device); time_kernels(*bt, reps, ms); });

@@ -52,9 +52,11 @@ public:
 	void apply(gfc_batch *bt, uint32_t n, size_t cap, uint32_t rep_b)
 	{
 		// a pool of packed-range bases tunes with packed plans among the
-		// candidates, whatever the RNS width of its representative base
+		// candidates, whatever the prime set of its representative base
 		const int packed = gfc_packed_range(rep_b, n);
-		const auto key = std::make_tuple(n, cap, packed ? 4 : gfc_width_for(rep_b, n), packed);
+		std::vector<int32_t> sets(cap);
+		ck(gfc_batch_prime_sets(bt, sets.data()), "prime_sets");
+		const auto key = std::make_tuple(n, cap, packed ? -1 : sets[0], packed);
 		{
 			std::lock_guard<std::mutex> l(mu_);
 			auto it = plans_.find(key);

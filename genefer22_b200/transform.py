@@ -63,6 +63,13 @@ class Batch:
         check(lib().gfc_batch_widths(self._h, _i32(w)))
         return w
 
+    def prime_sets(self) -> np.ndarray:
+        """Prime set per test with one digit per coefficient: 0 (two primes below
+        2^32), 3 (two below 2^31) or 1 (three below 2^31)."""
+        s = np.empty(self.count, dtype=np.int32)
+        check(lib().gfc_batch_prime_sets(self._h, _i32(s)))
+        return s
+
     def plan(self) -> int:
         return int(lib().gfc_batch_plan(self._h))
 

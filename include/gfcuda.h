@@ -233,8 +233,13 @@ int gfc_batch_set_all(gfc_batch *bt, size_t reg, const int32_t *in);
 int gfc_batch_set_plan(gfc_batch *bt, int lr);
 int gfc_batch_plan(const gfc_batch *bt);
 
-/* Per-test RNS width (2 or 3), into w[0..count-1]. */
+/* Per-test RNS width (2 or 3, or 4 with packed digits), into w[0..count-1]. */
 int gfc_batch_widths(const gfc_batch *bt, int32_t *w);
+
+/* Per-test prime set with one digit per coefficient, into s[0..count-1]: 0 two
+ * primes below 2^32, 3 two primes below 2^31, 1 three primes below 2^31 (the
+ * set the test takes when a batch with packed digits stops packing). */
+int gfc_batch_prime_sets(const gfc_batch *bt, int32_t *s);
 
 /* Waits for all enqueued work (see gfc_sync). */
 int gfc_batch_sync(gfc_batch *bt);

@@ -3,6 +3,8 @@
 Each test's residue must be the same alone, in an uneven batch and in the
 serving mix, and equal to the oracle's (restated transformCPUi32) where the
 oracle is run."""
+import json
+
 import numpy as np
 import pytest
 
@@ -106,6 +108,25 @@ def test_autotuner(tmp_path):
     tu2 = Autotuner(cache_path=path)
     bt = Batch([1_000_002] * 4, 15)
     assert tu2.tune(bt).lr == tu.cache[f"n15_c4_w0"]["lr"]
+
+
+def test_autotuner_keeps_prime_sets_and_kernels_apart(tmp_path):
+    """Batches of the two two-prime sets have entries of their own, and an entry
+    of another state of the kernels is measured again."""
+    path = str(tmp_path / "plans.json")
+    small, high = [1_000_002] * 4, [40_000_002] * 4         # sets 3 and 0 at n = 13
+    tu = Autotuner(cache_path=path, squarings=4, replays=2)
+    a, b = Batch(small, 13), Batch(high, 13)
+    assert list(a.prime_sets()) == [3] * 4 and list(b.prime_sets()) == [0] * 4
+    assert list(a.widths()) == list(b.widths()) == [2] * 4
+    ra, rb = tu.tune(a), tu.tune(b)
+    assert len(tu.cache) == 2 and ra.key() != rb.key()
+    assert Autotuner(cache_path=path).cache == tu.cache
+    with open(path, "w") as f:
+        json.dump({ra.key(): {"lr": 5, "us": {"5": 1.0}}}, f)
+    tu = Autotuner(cache_path=path, squarings=4, replays=2)
+    r = tu.tune(a)
+    assert set(r.us) != {5} and tu.cache[ra.key()]["lr"] == r.lr == a.plan()
 
 
 def test_uneven_batch_alone_vs_mix(oracle):
