@@ -44,6 +44,18 @@ bool query(cudaEvent_t e)
 	return false;
 }
 
+// Bases a pool is made and tuned with.  A pool of packed-range bases takes its
+// representative's like only; any other admits every base, and half of its
+// slots begin with one of three primes, so that its plan is chosen, by rule or
+// by measurement, for batches of both widths.
+std::vector<uint32_t> pool_bases(uint32_t n, size_t cap, uint32_t rep_b)
+{
+	std::vector<uint32_t> bases(cap, rep_b);
+	if (gfc_packed_range(rep_b, n) != 1)
+		for (size_t i = 1; i < cap; i += 2) bases[i] = 2000000000u;
+	return bases;
+}
+
 // Plans chosen by gfc_batch_tune per pool shape: (n, slots, prime set of the
 // representative base, packed range).
 class TuneCache
@@ -116,7 +128,7 @@ public:
 		: device_(device), B_(B)
 	{
 		ckc(cudaSetDevice(device), "cudaSetDevice");
-		std::vector<uint32_t> bases(cap, rep_b);
+		const std::vector<uint32_t> bases = pool_bases(n, cap, rep_b);
 		ck(gfc_batch_create(bases.data(), cap, n, 3, device, nullptr, &bt_), "batch_create");
 		if (tune) tc.apply(bt_, n, cap, rep_b);
 		ck(gfc_batch_reserve(bt_, (max_bits < B) ? B : max_bits), "reserve");
@@ -337,7 +349,7 @@ public:
 	void pretune(uint32_t n, size_t capacity, uint32_t rep_b) override
 	{
 		ckc(cudaSetDevice(device_), "cudaSetDevice");
-		std::vector<uint32_t> bases(capacity, rep_b);
+		const std::vector<uint32_t> bases = pool_bases(n, capacity, rep_b);
 		gfc_batch *bt = nullptr;
 		ck(gfc_batch_create(bases.data(), capacity, n, 3, device_, nullptr, &bt), "batch_create");
 		try { tune_.apply(bt, n, capacity, rep_b); }

@@ -13,7 +13,7 @@ from genefer22_b200 import genefer as gf
 from genefer22_b200.autotune import Autotuner, candidates
 from genefer22_b200.exponent import words_to_int
 from genefer22_b200.mixed import MixedBatch, run_alone, uneven_tests
-from genefer22_b200.serve import Server, pool_slot_bytes, serve_requests, slot_bytes, table_bytes
+from genefer22_b200.serve import Request, Server, pool_slot_bytes, serve_requests, slot_bytes, table_bytes
 
 pytestmark = pytest.mark.gpu
 
@@ -246,3 +246,13 @@ def test_native_server_reports_plans_and_stats():
     st = srv.stats
     assert st.blocks_run >= 2 and 1 <= st.pools_created and st.peak_bytes <= 4 * 10**9
     assert st.p50 <= st.p99
+
+
+def test_pool_plan_is_for_both_widths():
+    """A pool that admits any base is made for tests of two and three primes: at
+    n = 14 its default is the four-step plan also with 64 slots."""
+    B = 8
+    jobs = [gf.Job.prefix(b, 14, 2 * B) for b in (1_000_002, 1_999_999_998, 30_000_002)]
+    srv = Server(B=B, budget_bytes=8 * 10**9, capacity=lambda n: 64, tune=False, validate_group=2)
+    comps = srv.run([Request(i, j, 0.0) for i, j in enumerate(jobs)], timeout_s=120)
+    assert [c.plan for c in comps] == [3, 3, 3] and all(c.gl_ok for c in comps)
