@@ -208,6 +208,14 @@ def algorithmic(kind: int, widths: np.ndarray, n: int, lr: int):
     return float(np.sum(8 * N + 0 * W)), float(np.sum(W * (N / 2) * 2 * n + W * N))
 
 
+def butterfly_peak(widths: np.ndarray, sets: np.ndarray, probe) -> float:
+    """Radix-2 butterflies per second of the tests' primes (gfc_probe_int_throughput):
+    probe[3] for 31-bit ones (packed digits, prime sets 1 and 3), probe[2] for 32-bit
+    ones (set 0)."""
+    share31 = float(np.mean((widths == 4) | (sets != 0)))
+    return share31 * probe[3] + (1 - share31) * probe[2]
+
+
 def run_ours(args):
     import torch
     rank, world, local = dist_info()
@@ -302,8 +310,7 @@ def run_ours(args):
     achieved = abytes / (kms[dom] * 1e-3) / 1e9
     probe = (ctypes.c_double * 4)()
     L.gfc_probe_int_throughput(local, probe)
-    frac_w3 = float(np.mean(widths >= 3))       # 31-bit primes (3 or 4 of them) vs 32-bit (2)
-    bfly_peak = frac_w3 * probe[3] + (1 - frac_w3) * probe[2]
+    bfly_peak = butterfly_peak(widths, bt.prime_sets(), probe)
     traffic = None
     tj = os.path.join(ROOT, "profiles", "traffic.json")
     if os.path.exists(tj):
