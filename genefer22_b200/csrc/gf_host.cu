@@ -368,8 +368,8 @@ std::shared_ptr<DeviceTables> get_tables(int device, int n)
 	return t;
 }
 
-// The six-step twist factors of table t (2^t.n points, prime sets 0 and 1,
-// or set 2 when `packed`) for R = 2^lr rows, built on the device on first use.
+// The six-step twist factors of table t (2^t.n points, prime sets 0 and 1 (and
+// 3, set 1's first two), or set 2 when `packed`) for R = 2^lr rows, built on the device on first use.
 const TwistTables &get_twist(DeviceTables &t, bool packed, int lr)
 {
 	std::lock_guard<std::mutex> lock(t.tw_mu);
@@ -540,7 +540,6 @@ void set_smem(K kernel, size_t smem)
 	GFC_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
 }
 
-// `prep` only raises the kernel's shared-memory limit (done outside graph capture).
 // Streaming multiprocessors of the current device (cached per device).
 int sm_count()
 {
@@ -557,6 +556,7 @@ int sm_count()
 	return v;
 }
 
+// `prep` only raises the kernel's shared-memory limit (done outside graph capture).
 template <int SETS, int LOGN>
 void small_t(const Args &a, int grid, cudaStream_t s, bool prep)
 {
@@ -1075,7 +1075,7 @@ struct gfc_graph
 
 namespace {
 
-// Switches every test's descriptor between its own prime set (0 or 1, digits
+// Switches every test's descriptor between its own prime set (0, 1 or 3, digits
 // one per coefficient) and prime set 2 (packed digits).
 void set_packed(gfc_batch &bt, bool on)
 {
@@ -1209,7 +1209,6 @@ void launch_cluster(gfc_batch &bt, const Args &a, cudaStream_t s)
 	launch_cluster_n(bt.n, a, static_cast<int>(bt.count), bt.cluster_max, sets, s, false, nullptr);
 }
 
-// Raises shared-memory limits of the kernels the current plan uses.
 // Whether a six-step plan twists in its middle pass (every row then reads
 // the same C - 1 roots): where one direction of the row-pass root tables
 // (32 B per point of the packed transform, 24 B per point with a test on
@@ -1232,6 +1231,7 @@ bool twist_pays(const gfc_batch &bt)
 	return per_point * points >= (size_t(32) << 20);
 }
 
+// Raises shared-memory limits of the kernels the current plan uses.
 void prepare_plan(gfc_batch &bt)
 {
 	bt.twist = nullptr;

@@ -45,7 +45,8 @@ def check_ops(oracle, b, n, plan=None, seed=0, steps=4):
     assert np.array_equal(canon(t.getInt(), b), canon(o.getInt(), b)), "mul 2"
 
 
-# b values exercise both RNS widths: small b -> 2 primes, large b -> 3 primes
+# b values exercise both RNS widths: small b -> 2 primes (below 2^31 at every n here; two
+# primes below 2^32 are in test_prime_sets_gpu.py), large b -> 3 primes
 SMALL_B = 2 * 10**6
 LARGE_B = 2 * 10**9 - 2
 
@@ -79,8 +80,8 @@ def test_six_step_plan(oracle, n, plan, b):
 
 
 # Six-step plans whose middle pass twists the rows (the row-pass root tables of one direction
-# reach 32 MB: 8 B per point on the two-prime set, 24 B on the three-prime set), with 2^4 and
-# 2^5-row middle passes; the two-prime base at n = 21 keeps the plain rows.
+# reach 32 MB: 16 B per point on two 31-bit primes, 24 B on three), with 2^4 and 2^5-row middle
+# passes.
 @pytest.mark.parametrize("n,plan", [(21, 104), (22, 105)])
 @pytest.mark.parametrize("b", [SMALL_B // 4, LARGE_B])
 def test_twisted_six_step_plans(oracle, n, plan, b):

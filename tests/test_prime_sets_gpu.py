@@ -27,7 +27,7 @@ def test_edge_of_the_range(oracle, n, plan, step):
     b = top_base(n) + step
     t = Transform(b, n)
     t.batch.set_plan(plan)
-    assert t.width() == 2
+    assert t.width() == 2 and list(t.batch.prime_sets()) == [0 if step else 3]
     o = oracle.OracleTransform(b, n)
     d = np.full(1 << n, b // 2, dtype=np.int64)              # every product coefficient at its largest
     d[np.random.default_rng(n).integers(0, 1 << n, 9)] -= 1
@@ -37,6 +37,22 @@ def test_edge_of_the_range(oracle, n, plan, step):
         t.squareDup(dup)
         o.squareDup(dup)
     t.copy(1, 0); o.copy(1, 0)
+    t.mul(1); o.mul(1)
+    assert np.array_equal(gint.unbalance(t.getInt(), b), gint.unbalance(o.getInt(), b))
+
+
+# Set 0 twists its middle pass from n = 22 (8 B of row roots per point, 32 MB), set 3 from n = 21.
+@pytest.mark.parametrize("n,plan", [(21, 104), (22, 105), (22, 106), (23, 107)])
+@pytest.mark.parametrize("step", [0, 2])
+def test_largest_sizes_on_both_two_prime_sets(oracle, n, plan, step):
+    b = top_base(n) + step
+    t, o = Transform(b, n), oracle.OracleTransform(b, n)
+    t.batch.set_plan(plan)
+    assert list(t.batch.prime_sets()) == [0 if step else 3]
+    d = np.random.default_rng(n + plan).integers(-(b // 2), b // 2 + 1, 1 << n)
+    t.setInt(d); o.setInt(d)
+    t.copy(1, 0); o.copy(1, 0)
+    t.squareDup(True); o.squareDup(True)
     t.mul(1); o.mul(1)
     assert np.array_equal(gint.unbalance(t.getInt(), b), gint.unbalance(o.getInt(), b))
 
