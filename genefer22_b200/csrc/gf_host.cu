@@ -971,7 +971,10 @@ int default_small_plan(int n, size_t count, const int (&nset)[4])
 
 // The default packs a batch of at least this many tests whose bases all fit
 // (0: never): packed digits are faster from one test at n >= 16 (measured on
-// one B200 against the fastest unpacked plan).
+// one B200 against the fastest unpacked plan).  Below, no default packs, though
+// bases beyond set 3's range gain at n = 15 (one test 16.2 -> 13.5 us per squaring
+// with 203, 64 tests 68.2 -> 48.3 with 204) and in wide batches at n = 14 (128
+// tests 63.1 -> 46.8 with 203): gfc_batch_tune takes those plans.
 size_t packed_min_tests(int n)
 {
 	// a lone n = 19 test: the unpacked six-step 104 (35.5 us per squaring) beats
