@@ -146,3 +146,28 @@ def test_small_base_in_a_batch_made_without_one(oracle, n, plan, width):
         o.squareDup(bit)
     assert np.array_equal(gint.unbalance(bt.get(1), 2050), gint.unbalance(o.getInt(), 2050))
     bt.close()
+
+
+@pytest.mark.parametrize("n,plan", [(11, 0), (12, 0), (12, 1), (13, 3), (14, 1), (16, 4), (18, 103)])
+def test_admissions_across_the_sets(oracle, n, plan):
+    """A reserved batch on set 3 whose slots take tests of every set, and of set 3 again."""
+    wide = 1_999_999_998 if n <= 15 else 999_999_998
+    bt = Batch([1026, 2050, 4098], n)
+    bt.set_plan(plan)
+    bt.reserve(64)
+    bits = (True, False, True, True)
+    for bases, sets in (([top_base(n) + 2, wide, 1028], [0, 1, 3]), ([2052, top_base(n) + 4, wide - 2], [3, 0, 1]),
+                        ([1030, 2054, 4100], [3, 3, 3])):
+        for i, b in enumerate(bases):
+            bt.admit(i, b, np.array([0b1011], np.uint32), 4)
+        assert list(bt.prime_sets()) == sets
+        bt.square_exp(4)
+        for i, b in enumerate(bases):
+            o = oracle.OracleTransform(b, n)
+            o.set(1)
+            for bit in bits:
+                o.squareDup(bit)
+            assert np.array_equal(gint.unbalance(bt.get(i), b), gint.unbalance(o.getInt(), b)), (sets, i)
+        # dense digits through the same slots
+        _squared(bt, _load(oracle, bt, n), lambda: bt.square(True, 2), 2)
+    bt.close()
